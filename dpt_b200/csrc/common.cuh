@@ -363,6 +363,19 @@ __device__ __forceinline__ void red_add_v4(float* address, float a, float b, flo
                  : "memory");
 }
 
+// Two such reductions of a cell run's eight corner sums into the 32-byte record of cell
+// `pending` when the next sample's cell is another one: both under one predicate, so the
+// sample loop has no branch here.
+__device__ __forceinline__ void red_add_run(float* acc, int pending, int cell, const float* s)
+{
+    asm volatile("{\n\t.reg .pred ended;\n\t"
+                 "setp.ne.s32 ended, %9, %10;\n\t"
+                 "@ended red.global.add.v4.f32 [%8], {%0, %1, %2, %3};\n\t"
+                 "@ended red.global.add.v4.f32 [%8 + 16], {%4, %5, %6, %7};\n\t}" ::"f"(s[0]),
+                 "f"(s[1]), "f"(s[2]), "f"(s[3]), "f"(s[4]), "f"(s[5]), "f"(s[6]), "f"(s[7]),
+                 "l"(acc + 8 * (int64_t)pending), "r"(cell), "r"(pending));
+}
+
 // ------------------------------------------------------------ field access
 
 // Corner-replicated copies of the field, written by the pack kernel.
@@ -384,6 +397,19 @@ struct QuadF32 {
         v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
         v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
     }
+    // load_at of a cell below the last z plane when it is not the cell already held: both loads
+    // under one predicate, so the sample loop has no branch here and lanes that stay in their
+    // cell cost no L1 wavefront
+    __device__ __forceinline__ void refresh(int cell, int held, int, int, int, float* v) const
+    {
+        const float4* p = quad + cell;
+        asm("{\n\t.reg .pred moved;\n\t"
+            "setp.ne.s32 moved, %8, %9;\n\t"
+            "@moved ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%10];\n\t"
+            "@moved ld.global.nc.v4.f32 {%4, %5, %6, %7}, [%11];\n\t}"
+            : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3]), "+f"(v[4]), "+f"(v[5]), "+f"(v[6]), "+f"(v[7])
+            : "r"(cell), "r"(held), "l"(p), "l"(p + nx * ny));
+    }
     __device__ __forceinline__ void load(int lx, int ly, int lz, float* v) const
     {
         const int64_t plane = (int64_t)nx * ny;
@@ -403,6 +429,10 @@ struct PlainF32 {
     __device__ __forceinline__ void load_at(int, int lx, int ly, int lz, float* v) const
     {
         load(lx, ly, lz, v);
+    }
+    __device__ __forceinline__ void refresh(int cell, int held, int lx, int ly, int lz, float* v) const
+    {
+        if (cell != held) load(lx, ly, lz, v);
     }
     __device__ __forceinline__ void load(int lx, int ly, int lz, float* v) const
     {
@@ -557,7 +587,7 @@ __device__ __forceinline__ void inside_run(int samples, Inside inside_at, int& f
 // L1 hit it saves).
 template <class Field, bool kReuse = true>
 struct CellCache {
-    float v[8];
+    float v[8] = {};
     int cell = -1;
     __device__ __forceinline__ void fetch(const Field& f, int lx, int ly, int lz, int index)
     {
@@ -1088,6 +1118,29 @@ __device__ __forceinline__ f32x2 interior_fraction2(f32x2 p, f32x2* biased)
 __device__ __forceinline__ int biased_lo(f32x2 t) { return __float_as_int(lo2(t)) - kFloorBias; }
 __device__ __forceinline__ int biased_hi(f32x2 t) { return __float_as_int(hi2(t)) - kFloorBias; }
 
+// Flat cell index (z*ny + y)*nx + x from the three biased floors of one sample: the biases leave
+// the index off by a constant of the grid (mod 2^32), taken off once instead of once per axis.
+struct BiasedCells {
+    unsigned nx, ny, offset;
+    int shift_x, shift_y;
+    __device__ __forceinline__ void init(int nx_, int ny_)
+    {
+        nx = (unsigned)nx_;
+        ny = (unsigned)ny_;
+        offset = (unsigned)kFloorBias * (nx * ny + nx + 1u);
+        shift_x = __ffs(nx_) - 1;
+        shift_y = __ffs(ny_) - 1;
+    }
+    // kPow2: nx and ny are powers of two (shifts on the integer pipe)
+    template <bool kPow2>
+    __device__ __forceinline__ int at(float bx, float by, float bz) const
+    {
+        const unsigned x = __float_as_uint(bx), y = __float_as_uint(by), z = __float_as_uint(bz);
+        if constexpr (kPow2) return (int)((((z << shift_y) + y) << shift_x) + x - offset);
+        return (int)((z * ny + y) * nx + x - offset);
+    }
+};
+
 // Trilinear corner weights of two samples, (f0 f1) f2 per lane (corner_weights lane-wise).
 __device__ __forceinline__ void corner_weights2(f32x2 fx, f32x2 fy, f32x2 fz, f32x2* w, f32x2* ax_out = nullptr,
                                                 f32x2* ay_out = nullptr, f32x2* az_out = nullptr)
@@ -1108,20 +1161,45 @@ __device__ __forceinline__ void corner_weights2(f32x2 fx, f32x2 fy, f32x2 fz, f3
     if (az_out) *az_out = az;
 }
 
-// Interior slopes of two samples (slope32 with every mask 1), from each sample's eight corner
-// values: the twelve differences per sample are scalar, their combination lane-wise.
+// Scatter increments of two samples, ((factor f0) f1) f2 per corner: factor times the corner
+// weights with the factor taken into the x pair (14 products for the 20 of weights then
+// scaling, as many roundings each), the last product flushing results below the normal range.
+__device__ __forceinline__ void scatter_increments2(f32x2 factor, f32x2 fx, f32x2 fy, f32x2 fz, f32x2* inc)
+{
+    const f32x2 one = splat2(1.0f);
+    const f32x2 ay = sub2(one, fy), az = sub2(one, fz);
+    const f32x2 px = mul2(factor, fx), qx = mul2(factor, sub2(one, fx));
+    const f32x2 p00 = mul2(qx, ay), p10 = mul2(px, ay), p01 = mul2(qx, fy), p11 = mul2(px, fy);
+    inc[0] = mul_ftz2(p00, az);
+    inc[1] = mul_ftz2(p10, az);
+    inc[2] = mul_ftz2(p01, az);
+    inc[3] = mul_ftz2(p11, az);
+    inc[4] = mul_ftz2(p00, fz);
+    inc[5] = mul_ftz2(p10, fz);
+    inc[6] = mul_ftz2(p01, fz);
+    inc[7] = mul_ftz2(p11, fz);
+}
+
+// The twelve corner differences of one cell that its interior slopes combine: along x
+// (10, 32, 54, 76), along y (20, 31, 64, 75), along z (40, 51, 62, 73).
+__device__ __forceinline__ void corner_differences(const float* v, float* d)
+{
+    d[0] = v[1] - v[0]; d[1] = v[3] - v[2]; d[2] = v[5] - v[4]; d[3] = v[7] - v[6];
+    d[4] = v[2] - v[0]; d[5] = v[3] - v[1]; d[6] = v[6] - v[4]; d[7] = v[7] - v[5];
+    d[8] = v[4] - v[0]; d[9] = v[5] - v[1]; d[10] = v[6] - v[2]; d[11] = v[7] - v[3];
+}
+
+// Interior slopes of two samples (slope32 with every mask 1) from the corner differences of
+// their cells (one sample per lane).
 __device__ __forceinline__ void slope2(f32x2 fx, f32x2 fy, f32x2 fz, f32x2 ax, f32x2 ay, f32x2 az,
                                        const float* u, const float* v, f32x2* g)
 {
-    const f32x2 d10 = pack2(u[1] - u[0], v[1] - v[0]), d32 = pack2(u[3] - u[2], v[3] - v[2]);
-    const f32x2 d54 = pack2(u[5] - u[4], v[5] - v[4]), d76 = pack2(u[7] - u[6], v[7] - v[6]);
-    g[0] = fma2(fz, fma2(fy, d76, mul2(ay, d54)), mul2(az, fma2(fy, d32, mul2(ay, d10))));
-    const f32x2 d20 = pack2(u[2] - u[0], v[2] - v[0]), d31 = pack2(u[3] - u[1], v[3] - v[1]);
-    const f32x2 d64 = pack2(u[6] - u[4], v[6] - v[4]), d75 = pack2(u[7] - u[5], v[7] - v[5]);
-    g[1] = fma2(fz, fma2(fx, d75, mul2(ax, d64)), mul2(az, fma2(fx, d31, mul2(ax, d20))));
-    const f32x2 d40 = pack2(u[4] - u[0], v[4] - v[0]), d51 = pack2(u[5] - u[1], v[5] - v[1]);
-    const f32x2 d62 = pack2(u[6] - u[2], v[6] - v[2]), d73 = pack2(u[7] - u[3], v[7] - v[3]);
-    g[2] = fma2(fy, fma2(fx, d73, mul2(ax, d62)), mul2(ay, fma2(fx, d51, mul2(ax, d40))));
+    f32x2 d[12];
+#pragma unroll
+    for (int k = 0; k < 12; ++k) d[k] = pack2(u[k], v[k]);
+    g[0] = fma2(fz, fma2(fy, d[3], mul2(ay, d[2])), mul2(az, fma2(fy, d[1], mul2(ay, d[0]))));
+    g[1] = fma2(fz, fma2(fx, d[7], mul2(ax, d[6])), mul2(az, fma2(fx, d[5], mul2(ax, d[4]))));
+    g[2] = fma2(fy, fma2(fx, d[11], mul2(ax, d[10])), mul2(ay, fma2(fx, d[9], mul2(ax, d[8]))));
 }
 
 // Per-block staging of the view's pose (12 doubles) and panel record.

@@ -22,12 +22,20 @@
 
 #include "launch.h"
 
-#ifndef DPT_FORWARD_REUSE
-#define DPT_FORWARD_REUSE 1  // FP32 forward: reload the corners only when the sample enters another cell
+// Resident blocks per SM the register allocation must allow.  FP32: 32 views of the 256^3 /
+// 512^2 / S = 1024 scan take 12.4 ms at eight blocks (62 registers), 12.8 at nine (56).
+#ifndef DPT_FORWARD_MIN_BLOCKS_F32
+#define DPT_FORWARD_MIN_BLOCKS_F32 8
 #endif
 
 namespace dpt {
 namespace {
+
+template <int kArith>
+constexpr int forward_min_blocks()
+{
+    return kArith == DPT_ARITH_F32 ? DPT_FORWARD_MIN_BLOCKS_F32 : 0;
+}
 
 // FP32 sample of the field at grid point (x, y, z): zero outside the half-cell support.
 template <class Field>
@@ -125,7 +133,7 @@ __device__ __forceinline__ void forward_tile(const RayArgs& a, const Field& f, O
                         at(i, x, y, z);
                         return x >= 0.0f && x < dims.mx && y >= 0.0f && y < dims.my && z >= 0.0f && z < dims.mz;
                     }, ifirst, ilast);
-                    CellCache<Field, DPT_FORWARD_REUSE != 0> cache;
+                    CellCache<Field> cache;
                     auto add = [&](Axis32 X, Axis32 Y, Axis32 Z) {
                         cache.fetch(f, X.lower, Y.lower, Z.lower, (Z.lower * dims.ny + Y.lower) * dims.nx + X.lower);
                         float w[8];
@@ -139,8 +147,48 @@ __device__ __forceinline__ void forward_tile(const RayArgs& a, const Field& f, O
                     };
                     const int split = min(ifirst, last + 1);
                     for (int i = first; i < split; ++i) margin(i);
-#pragma unroll 4
-                    for (int i = ifirst; i <= ilast; ++i) {
+                    int i = ifirst;
+                    // Samples i and i + 1 of the interior run at once: positions, floors and corner
+                    // weights lane-wise (see "packed FP32 pairs" in common.cuh), the corners
+                    // reloaded under a predicate, the ray sum serial in sample order, so the total
+                    // is the one the scalar samples form.  The kernel is bound by issue slots: 32
+                    // views of the 256^3 / 512^2 / S = 1024 scan 13.9 -> 12.4 ms (54 -> 44 thread
+                    // instructions per sample).  The floors need coordinates, and the exact
+                    // sample parameters i + 0.5, below 2^23.
+                    if (dims.packed && S <= (1 << 23)) {
+                        f32x2 ip = pack2((float)i + 0.5f, (float)i + 1.5f);
+                        BiasedCells cells;
+                        cells.init(dims.nx, dims.ny);
+                        for (; i + 1 <= ilast; i += 2) {
+                            const f32x2 position = fma2(ip, splat2(step), splat2(iv.lower));
+                            ip = add2(ip, splat2(2.0f));
+                            const f32x2 x = fma2(position, splat2(d[0]), splat2(o[0]));
+                            const f32x2 y = fma2(position, splat2(d[1]), splat2(o[1]));
+                            const f32x2 z = fma2(position, splat2(d[2]), splat2(o[2]));
+                            f32x2 bx, by, bz;
+                            const f32x2 fx = interior_fraction2(x, &bx);
+                            const f32x2 fy = interior_fraction2(y, &by);
+                            const f32x2 fz = interior_fraction2(z, &bz);
+                            f32x2 w[8];
+                            corner_weights2(fx, fy, fz, w);
+                            float w0[8], w1[8];
+#pragma unroll
+                            for (int c = 0; c < 8; ++c) {
+                                w0[c] = lo2(w[c]);
+                                w1[c] = hi2(w[c]);
+                            }
+                            const int lx0 = biased_lo(bx), ly0 = biased_lo(by), lz0 = biased_lo(bz);
+                            const int lx1 = biased_hi(bx), ly1 = biased_hi(by), lz1 = biased_hi(bz);
+                            const int cell0 = cells.at<false>(lo2(bx), lo2(by), lo2(bz));
+                            const int cell1 = cells.at<false>(hi2(bx), hi2(by), hi2(bz));
+                            f.refresh(cell0, cache.cell, lx0, ly0, lz0, cache.v);
+                            total = total + interpolate(w0, cache.v);
+                            f.refresh(cell1, cell0, lx1, ly1, lz1, cache.v);
+                            total = total + interpolate(w1, cache.v);
+                            cache.cell = cell1;
+                        }
+                    }
+                    for (; i <= ilast; ++i) {
                         float x, y, z;
                         at(i, x, y, z);
                         add(interior_axis(x), interior_axis(y), interior_axis(z));
@@ -404,7 +452,8 @@ __device__ __forceinline__ void forward_tile(const RayArgs& a, const Field& f, O
 }
 
 template <int kArith, class Field, typename Out>
-__global__ void __launch_bounds__(kForwardBlock) k_forward(RayArgs a, Field f, Out* __restrict__ image)
+__global__ void __launch_bounds__(kForwardBlock, forward_min_blocks<kArith>())
+    k_forward(RayArgs a, Field f, Out* __restrict__ image)
 {
     __shared__ ViewShared vs;
     __shared__ float4 run_sums[kArith == DPT_ARITH_F32C ? kRunSumTable + 1 : 1];

@@ -32,6 +32,11 @@
 #ifndef DPT_VJP_MIN_BLOCKS_F32
 #define DPT_VJP_MIN_BLOCKS_F32 6
 #endif
+// The FP32 volume scatter alone (per 32 views of the full scan): 16.2 ms at six blocks (80
+// registers), 16.3 at eight (64).
+#ifndef DPT_VJP_MIN_BLOCKS_F32_VOLUME
+#define DPT_VJP_MIN_BLOCKS_F32_VOLUME 6
+#endif
 #ifndef DPT_VJP_MIN_BLOCKS_F32C
 #define DPT_VJP_MIN_BLOCKS_F32C 8
 #endif
@@ -50,11 +55,11 @@
 #ifndef DPT_VJP_MIN_BLOCKS_F32C_JOINT
 #define DPT_VJP_MIN_BLOCKS_F32C_JOINT 8
 #endif
-// The FP32 forward that stores the pose moments: 289.1 ms per full scan at six blocks (80
-// registers, 84 bytes spilled), 289.5 at five (88 registers, none spilled), 316.0 at seven;
-// the occupancy does not matter where the FP32 pipe binds.
+// The FP32 forward that stores the pose moments (per 32 views of the full scan): 24.1 ms at
+// four and five blocks (none spilled), 25.0 at six (80 registers, 76 bytes spilled), 25.8 at
+// seven; the occupancy does not matter where the FP32 pipe binds.
 #ifndef DPT_VJP_MIN_BLOCKS_F32_MOMENTS
-#define DPT_VJP_MIN_BLOCKS_F32_MOMENTS 6
+#define DPT_VJP_MIN_BLOCKS_F32_MOMENTS 5
 #endif
 // Strict FP64: the full-scan joint VJP (launches of two views) measured 86.7 ms per 32 views
 // at three blocks (160 registers), 84.3 at four (128, 68 bytes spilled), 83.2 at five (96,
@@ -148,20 +153,27 @@ struct MomentArgs {
     float* image;    // kStoreMoments: the forward image (FP32)
 };
 
+template <int kArith, bool kVol, bool kPose, int kMoments>
+constexpr int vjp_min_blocks()
+{
+    if (kArith == DPT_ARITH_F32C)
+        return kMoments == kStoreMoments ? DPT_VJP_MIN_BLOCKS_F32C_FORWARD
+             : kVol && kPose             ? DPT_VJP_MIN_BLOCKS_F32C_JOINT
+                                         : DPT_VJP_MIN_BLOCKS_F32C;
+    if (kArith == DPT_ARITH_F32)
+        return kMoments == kStoreMoments ? DPT_VJP_MIN_BLOCKS_F32_MOMENTS
+             : !kPose                    ? DPT_VJP_MIN_BLOCKS_F32_VOLUME
+                                         : DPT_VJP_MIN_BLOCKS_F32;
+    if (kArith == DPT_ARITH_F64) return DPT_VJP_MIN_BLOCKS_F64;
+    return kArith == DPT_ARITH_CELLS ? DPT_VJP_MIN_BLOCKS_CELLS : DPT_VJP_MIN_BLOCKS_FP64_OTHER;
+}
+
 // kPow2: nx and ny are powers of two, so the interior pairs form their flat cell index with
 // shifts (integer pipe) instead of two multiply-adds on the FP32 pipe, which binds the
 // moment-storing forward (full scan at 256^3: 289.0 -> 283.7 ms, the same values).
 template <int kArith, class Field, bool kVol, bool kPose, typename Seed, int kMoments = kJointMoments,
           bool kPow2 = false>
-__global__ void __launch_bounds__(kVjpBlock, kArith == DPT_ARITH_F32C
-                                                  ? (kMoments == kStoreMoments ? DPT_VJP_MIN_BLOCKS_F32C_FORWARD
-                                                     : (kVol && kPose)             ? DPT_VJP_MIN_BLOCKS_F32C_JOINT
-                                                                                   : DPT_VJP_MIN_BLOCKS_F32C)
-                                                  : kArith == DPT_ARITH_F32 ? (kMoments == kStoreMoments ? DPT_VJP_MIN_BLOCKS_F32_MOMENTS
-                                                                                                         : DPT_VJP_MIN_BLOCKS_F32)
-                                                  : kArith == DPT_ARITH_F64   ? DPT_VJP_MIN_BLOCKS_F64
-                                                  : kArith == DPT_ARITH_CELLS ? DPT_VJP_MIN_BLOCKS_CELLS
-                                                                              : DPT_VJP_MIN_BLOCKS_FP64_OTHER)
+__global__ void __launch_bounds__(kVjpBlock, vjp_min_blocks<kArith, kVol, kPose, kMoments>())
     k_vjp(RayArgs a, Field f, const Seed* __restrict__ cot,
                                                 int mode, float* __restrict__ acc,
                                                 double* __restrict__ partials, MomentArgs ma)
@@ -235,7 +247,9 @@ __global__ void __launch_bounds__(kVjpBlock, kArith == DPT_ARITH_F32C
                     int pending = -1;
                     CellCache<Field, kVjpReuse> cache;
                     auto position_at = [&](int i) { return fmaf((float)i + 0.5f, step, iv.lower); };
-                    const int shift_x = kPow2 ? __ffs(dims.nx) - 1 : 0, shift_y = kPow2 ? __ffs(dims.ny) - 1 : 0;
+                    BiasedCells cells;
+                    cells.init(dims.nx, dims.ny);
+                    int held = -1;  // the cell of the pair loop's corners
                     const float inverse_samples = 1.0f / (float)S;
                     // One midpoint.  mode 0: general (support and finiteness tested); 1: on the
                     // inside run (both known to pass); 2: on the interior run (no clamp active,
@@ -353,42 +367,48 @@ __global__ void __launch_bounds__(kVjpBlock, kArith == DPT_ARITH_F32C
                     // Samples i and i + 1 of the interior run, lane-wise where the arithmetic is
                     // (see "packed FP32 pairs" in common.cuh); the serial sums take sample i,
                     // then sample i + 1, so every moment, increment and run sum is the value
-                    // the two visits of mode 2 form.  `ip` holds (i + 0.5, i + 1.5).
+                    // the two visits of mode 2 form.  `ip` holds (i + 0.5, i + 1.5).  Positions and
+                    // coordinates stay scalar (a packed operand of a per-ray value takes two
+                    // registers).  The corners reload, and a finished run flushes, under a
+                    // predicate instead of a branch: 32 views of the 256^3 / 512^2 / S = 1024
+                    // scan take 39.0 ms jointly (51.2 before), 24.1 storing the moments (25.2),
+                    // 16.2 scattering (16.3); 512^3 at 0.5 mm, 16 views: 14.4 (15.6) and 29.0 (31.3).
                     auto visit_pair = [&](int i, f32x2 ip, auto bounded_tag, auto pow2_tag) {
                         (void)bounded_tag;
-                        const f32x2 position = fma2(ip, splat2(step), splat2(iv.lower));
-                        const f32x2 x = fma2(position, splat2(d[0]), splat2(o[0]));
-                        const f32x2 y = fma2(position, splat2(d[1]), splat2(o[1]));
-                        const f32x2 z = fma2(position, splat2(d[2]), splat2(o[2]));
+                        const float q0 = fmaf(lo2(ip), step, iv.lower), q1 = fmaf(hi2(ip), step, iv.lower);
+                        const f32x2 position = pack2(q0, q1);
+                        const f32x2 x = pack2(fmaf(q0, d[0], o[0]), fmaf(q1, d[0], o[0]));
+                        const f32x2 y = pack2(fmaf(q0, d[1], o[1]), fmaf(q1, d[1], o[1]));
+                        const f32x2 z = pack2(fmaf(q0, d[2], o[2]), fmaf(q1, d[2], o[2]));
                         f32x2 bx, by, bz;
                         const f32x2 fx = interior_fraction2(x, &bx);
                         const f32x2 fy = interior_fraction2(y, &by);
                         const f32x2 fz = interior_fraction2(z, &bz);
-                        f32x2 w[8], ax, ay, az;
-                        corner_weights2(fx, fy, fz, w, &ax, &ay, &az);
                         const int lx0 = biased_lo(bx), ly0 = biased_lo(by), lz0 = biased_lo(bz);
                         const int lx1 = biased_hi(bx), ly1 = biased_hi(by), lz1 = biased_hi(bz);
-                        int cell0, cell1;
-                        if constexpr (kPow2) {
-                            cell0 = (((lz0 << shift_y) + ly0) << shift_x) + lx0;
-                            cell1 = (((lz1 << shift_y) + ly1) << shift_x) + lx1;
-                        } else {
-                            cell0 = (lz0 * dims.ny + ly0) * dims.nx + lx0;
-                            cell1 = (lz1 * dims.ny + ly1) * dims.nx + lx1;
-                        }
+                        const int cell0 = cells.at<kPow2>(lo2(bx), lo2(by), lo2(bz));
+                        const int cell1 = cells.at<kPow2>(hi2(bx), hi2(by), hi2(bz));
+                        f32x2 inc[8];
                         if (kPose) {
-                            float u[8], v[8];
-                            f.load_at(cell0, lx0, ly0, lz0, u);
-                            f.load_at(cell1, lx1, ly1, lz1, v);
+                            f32x2 w[8], ax, ay, az;
+                            corner_weights2(fx, fy, fz, w, &ax, &ay, &az);
                             float wu[8], wv[8];
 #pragma unroll
                             for (int c = 0; c < 8; ++c) {
                                 wu[c] = lo2(w[c]);
                                 wv[c] = hi2(w[c]);
+                                if (kVol) inc[c] = mul_ftz2(splat2(vf), w[c]);
                             }
-                            const float value0 = interpolate(wu, u), value1 = interpolate(wv, v);
+                            float du[12], dv[12];
+                            f.refresh(cell0, held, lx0, ly0, lz0, cache.v);
+                            const float value0 = interpolate(wu, cache.v);
+                            corner_differences(cache.v, du);
+                            f.refresh(cell1, cell0, lx1, ly1, lz1, cache.v);
+                            const float value1 = interpolate(wv, cache.v);
+                            corner_differences(cache.v, dv);
+                            held = cell1;
                             f32x2 gs[3];
-                            slope2(fx, fy, fz, ax, ay, az, u, v, gs);
+                            slope2(fx, fy, fz, ax, ay, az, du, dv, gs);
                             mean = mean + value0;
                             mean = mean + value1;
                             const float p0 = lo2(position), p1 = hi2(position);
@@ -413,28 +433,19 @@ __global__ void __launch_bounds__(kVjpBlock, kArith == DPT_ARITH_F32C
                             su = fmaf(hi2(alpha), hi2(along), su);
                         }
                         if (kVol) {
-                            // bounded increments only (the pair loop runs for bounded rays)
-                            f32x2 inc[8];
+                            // bounded increments only (the pair loop runs for bounded rays).  The
+                            // sums restart by a factor 0 (finite sums: 0 s + x = x) instead of a
+                            // branch: lanes of a warp change cells at different samples
+                            if constexpr (!kPose) scatter_increments2(splat2(vf), fx, fy, fz, inc);
+                            red_add_run(acc, pending, cell0, cs);
+                            const float keep0 = cell0 == pending ? 1.0f : 0.0f;
 #pragma unroll
-                            for (int c = 0; c < 8; ++c) inc[c] = mul_ftz2(splat2(vf), w[c]);
-                            if (cell0 != pending) {
-                                if (pending >= 0) flush_run(pending, cs);
-                                pending = cell0;
+                            for (int c = 0; c < 8; ++c) cs[c] = fmaf(cs[c], keep0, lo2(inc[c]));
+                            red_add_run(acc, cell0, cell1, cs);
+                            const float keep1 = cell1 == cell0 ? 1.0f : 0.0f;
 #pragma unroll
-                                for (int c = 0; c < 8; ++c) cs[c] = lo2(inc[c]);
-                            } else {
-#pragma unroll
-                                for (int c = 0; c < 8; ++c) cs[c] = cs[c] + lo2(inc[c]);
-                            }
-                            if (cell1 != pending) {
-                                flush_run(pending, cs);
-                                pending = cell1;
-#pragma unroll
-                                for (int c = 0; c < 8; ++c) cs[c] = hi2(inc[c]);
-                            } else {
-#pragma unroll
-                                for (int c = 0; c < 8; ++c) cs[c] = cs[c] + hi2(inc[c]);
-                            }
+                            for (int c = 0; c < 8; ++c) cs[c] = fmaf(cs[c], keep1, hi2(inc[c]));
+                            pending = cell1;
                         }
                     };
                     auto march = [&](auto bounded_tag, auto pow2_tag) {
@@ -460,8 +471,15 @@ __global__ void __launch_bounds__(kVjpBlock, kArith == DPT_ARITH_F32C
                         int i = ifirst;
                         // the pair floors need interior coordinates below 2^23, and the pair
                         // scatter bounded increments
-                        if (dims.packed && (!kVol || decltype(bounded_tag)::value)) {
+                        if (dims.packed && S <= (1 << 23) && (!kVol || decltype(bounded_tag)::value)) {
                             f32x2 ip = pack2((float)i + 0.5f, (float)i + 1.5f);
+                            if (kVol && pending < 0 && i < ilast) {
+                                const float position = position_at(i);
+                                const Axis32 X = interior_axis(fmaf(position, d[0], o[0]));
+                                const Axis32 Y = interior_axis(fmaf(position, d[1], o[1]));
+                                const Axis32 Z = interior_axis(fmaf(position, d[2], o[2]));
+                                pending = (Z.lower * dims.ny + Y.lower) * dims.nx + X.lower;
+                            }
                             for (; i + 1 <= ilast; i += 2) {
                                 visit_pair(i, ip, bounded_tag, pow2_tag);
                                 ip = add2(ip, splat2(2.0f));
