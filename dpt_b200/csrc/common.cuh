@@ -527,6 +527,21 @@ __device__ __forceinline__ void slope64(double fx, double fy, double fz, const d
     g[2] = sz * fma(fy, dz1, ay * dz0);
 }
 
+// slope64 inside the grid, where every mask is 1 (a factor 1 changes nothing).
+__device__ __forceinline__ void interior_slope64(double fx, double fy, double fz, const double* v, double* g)
+{
+    const double ax = 1.0 - fx, ay = 1.0 - fy, az = 1.0 - fz;
+    const double dx0 = fma(fy, v[3] - v[2], ay * (v[1] - v[0]));
+    const double dx1 = fma(fy, v[7] - v[6], ay * (v[5] - v[4]));
+    const double dy0 = fma(fx, v[3] - v[1], ax * (v[2] - v[0]));
+    const double dy1 = fma(fx, v[7] - v[5], ax * (v[6] - v[4]));
+    const double dz0 = fma(fx, v[5] - v[1], ax * (v[4] - v[0]));
+    const double dz1 = fma(fx, v[7] - v[3], ax * (v[6] - v[2]));
+    g[0] = fma(fz, dx1, az * dx0);
+    g[1] = fma(fz, dy1, az * dy0);
+    g[2] = fma(fy, dz1, ay * dz0);
+}
+
 // Grid bounds used by every sample (computed once per thread).
 struct FieldDims {
     int nx, ny, nz;
@@ -626,6 +641,20 @@ __device__ __forceinline__ Axis32 interior_axis(float p)
     Axis32 r;
     r.lower = __float2int_rd(p);
     r.fraction = p - (float)r.lower;
+    return r;
+}
+
+// The same for an FP64 coordinate, 0 <= p < 2^31, on the FP64 pipe alone: p + 2^52 rounded toward
+// -inf is 2^52 + floor(p) exactly, its low word is floor(p) and taking 2^52 off again gives
+// floor(p) exactly (the conversions and the clamp of axis64 are three XU and two FP64
+// instructions more).
+__device__ __forceinline__ Axis64 interior_axis64(double p)
+{
+    constexpr double kMagic = 4503599627370496.0;  // 2^52
+    const double t = __dadd_rd(p, kMagic);
+    Axis64 r;
+    r.lower = __double2loint(t);
+    r.fraction = p - (t - kMagic);
     return r;
 }
 

@@ -36,8 +36,8 @@ cudaError_t launch_vjp(const dpt_problem& p, const RayArgs& a, const void* packe
                        const void* cotangent, int flags, float* accumulator, double* partials,
                        cudaStream_t stream);
 cudaError_t launch_forward_moments(const dpt_problem& p, const RayArgs& a, const void* packed,
-                                   float* image, float* moments, int64_t stride, cudaStream_t stream);
-cudaError_t launch_pose_from_moments(const dpt_problem& p, const RayArgs& a, const float* moments,
+                                   void* image, void* moments, int64_t stride, cudaStream_t stream);
+cudaError_t launch_pose_from_moments(const dpt_problem& p, const RayArgs& a, const void* moments,
                                      int64_t stride, const void* cotangent, int flags,
                                      double* partials, cudaStream_t stream);
 cudaError_t launch_finish_pose(int view_begin, int view_count, int tiles, int components,

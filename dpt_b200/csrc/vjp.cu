@@ -61,12 +61,15 @@
 #ifndef DPT_VJP_MIN_BLOCKS_F32_MOMENTS
 #define DPT_VJP_MIN_BLOCKS_F32_MOMENTS 5
 #endif
-// Strict FP64: the full-scan joint VJP (launches of two views) measured 86.7 ms per 32 views
-// at three blocks (160 registers), 84.3 at four (128, 68 bytes spilled), 83.2 at five (96,
-// 376 bytes spilled to L1).  The cell-Gauss joint VJP: 61.5 ms per 32 views at three blocks,
-// 59.3 at four, 66.0 at five.  The mixed and fast forms keep three.
+// Strict FP64, 16 views of the full scan: the pose pass 23.0 ms at four blocks (128 registers,
+// 212 bytes spilled), 25.1 at five (96, 452 bytes); the volume scatter 15.2 ms at six blocks
+// (80 registers), 15.8 at seven (72).  The cell-Gauss joint VJP: 61.5 ms per 32 views at three
+// blocks, 59.3 at four, 66.0 at five.  The mixed and fast forms keep three.
 #ifndef DPT_VJP_MIN_BLOCKS_F64
-#define DPT_VJP_MIN_BLOCKS_F64 5
+#define DPT_VJP_MIN_BLOCKS_F64 4
+#endif
+#ifndef DPT_VJP_MIN_BLOCKS_F64_VOLUME
+#define DPT_VJP_MIN_BLOCKS_F64_VOLUME 6
 #endif
 #ifndef DPT_VJP_MIN_BLOCKS_CELLS
 #define DPT_VJP_MIN_BLOCKS_CELLS 4
@@ -146,11 +149,14 @@ constexpr int kJointMoments = 0, kStoreMoments = 1, kLoadMoments = 2;
 // compensation, G[3], H[3] and whether H is the cell-run sum (to divide by S) or already
 // alpha-weighted (per-sample form)
 constexpr int kMomentWords = 9;
+// the words (and the image) are FP32, or FP64 for the strict FP64 arithmetic
+template <int kArith>
+using MomentWord = std::conditional_t<kArith == DPT_ARITH_F64, double, float>;
 
 struct MomentArgs {
-    float* moments;  // kMomentWords x stride FP32, word k of ray r at k * stride + r
+    void* moments;   // kMomentWords x stride words, word k of ray r at k * stride + r
     int64_t stride;  // rays of the call
-    float* image;    // kStoreMoments: the forward image (FP32)
+    void* image;     // kStoreMoments: the forward image
 };
 
 template <int kArith, bool kVol, bool kPose, int kMoments>
@@ -164,7 +170,7 @@ constexpr int vjp_min_blocks()
         return kMoments == kStoreMoments ? DPT_VJP_MIN_BLOCKS_F32_MOMENTS
              : !kPose                    ? DPT_VJP_MIN_BLOCKS_F32_VOLUME
                                          : DPT_VJP_MIN_BLOCKS_F32;
-    if (kArith == DPT_ARITH_F64) return DPT_VJP_MIN_BLOCKS_F64;
+    if (kArith == DPT_ARITH_F64) return kPose ? DPT_VJP_MIN_BLOCKS_F64 : DPT_VJP_MIN_BLOCKS_F64_VOLUME;
     return kArith == DPT_ARITH_CELLS ? DPT_VJP_MIN_BLOCKS_CELLS : DPT_VJP_MIN_BLOCKS_FP64_OTHER;
 }
 
@@ -179,8 +185,9 @@ __global__ void __launch_bounds__(kVjpBlock, vjp_min_blocks<kArith, kVol, kPose,
                                                 double* __restrict__ partials, MomentArgs ma)
 {
     static_assert(kMoments == kJointMoments ||
-                      ((kArith == DPT_ARITH_F32 || kArith == DPT_ARITH_F32C) && !kVol && kPose),
-                  "split pose moments: FP32 or compensated arithmetic, pose only");
+                      ((kArith == DPT_ARITH_F32 || kArith == DPT_ARITH_F32C || kArith == DPT_ARITH_F64) && !kVol && kPose),
+                  "split pose moments: FP32, compensated or strict FP64 arithmetic, pose only");
+    using Word = MomentWord<kArith>;
     __shared__ ViewShared vs;
     __shared__ double warp_sums[kVjpBlock / 32][12];
     __shared__ float4 run_sums[kArith == DPT_ARITH_F32C && kMoments != kLoadMoments ? kRunSumTable + 1 : 1];
@@ -206,8 +213,8 @@ __global__ void __launch_bounds__(kVjpBlock, vjp_min_blocks<kArith, kVol, kPose,
 #pragma unroll
     for (int k = 0; k < 12; ++k) g[k] = 0.0;
     int bits = 0;
-    float stored[kMoments == kStoreMoments ? kMomentWords : 1] = {};
-    float stored_image = 0.0f;
+    Word stored[kMoments == kStoreMoments ? kMomentWords : 1] = {};
+    Word stored_image = 0;
 
     if (active) {
         double source[3], end[3];
@@ -491,7 +498,7 @@ __global__ void __launch_bounds__(kVjpBlock, vjp_min_blocks<kArith, kVol, kPose,
                     }
                     };
                     if constexpr (kMoments == kLoadMoments) {
-                        const float* m = ma.moments + ray_index;
+                        const float* m = static_cast<const float*>(ma.moments) + ray_index;
                         mean = m[0];
 #pragma unroll
                         for (int k = 0; k < 3; ++k) {
@@ -859,7 +866,18 @@ __global__ void __launch_bounds__(kVjpBlock, vjp_min_blocks<kArith, kVol, kPose,
                             }
                         }
                     };
-                    if (!moderate(r.origin, r.direction)) {
+                    bool trailing_zero = false;
+                    if constexpr (kMoments == kLoadMoments) {
+                        const double* m = static_cast<const double*>(ma.moments) + ray_index;
+                        mean = m[0];
+#pragma unroll
+                        for (int k = 0; k < 3; ++k) {
+                            dO[k] = m[(1 + k) * ma.stride];
+                            dD[k] = m[(4 + k) * ma.stride];
+                        }
+                        sl = m[7 * ma.stride];
+                        su = m[8 * ma.stride];
+                    } else if (!moderate(r.origin, r.direction)) {
                         for (int i = 0; i < S; ++i) visit(i, false);
                     } else {
                         int first, last;
@@ -868,10 +886,90 @@ __global__ void __launch_bounds__(kVjpBlock, vjp_min_blocks<kArith, kVol, kPose,
                             point_at(i, position, p);
                             return inside(p[0], p[1], p[2], dims.nx, dims.ny, dims.nz);
                         }, first, last);
-                        for (int i = first; i <= last; ++i) visit(i, true);
+                        // every rounded increment is at most |vf| (1 + 2^-50) in magnitude, so the
+                        // sum of a run of up to 2^31 of them stays finite in FP32
+                        const bool bounded = fabs(vf) <= 1e28;
+                        int ifirst = last + 1, ilast = last;
+                        if (!kVol || bounded)
+                            interior_run(first, last, [&](int i) {
+                                double position, p[3];
+                                point_at(i, position, p);
+                                return p[0] >= 0.0 && p[0] < mx && p[1] >= 0.0 && p[1] < my && p[2] >= 0.0 && p[2] < mz;
+                            }, ifirst, ilast);
+                        const int split = min(ifirst, last + 1);
+                        for (int i = first; i < split; ++i) visit(i, true);
+                        // The interior run: no clamp, slope masks 1, no test of an increment, no
+                        // conversion of a coordinate; corners reload and run sums restart without
+                        // a branch as in the FP32 pairs.  16 views of the 256^3 / 512^2 / S = 1024
+                        // scan: pose 27.3 -> 23.0 ms (FP64 pipe 69 %), scatter 17.9 -> 15.2 (its
+                        // eight roundings to FP32 per sample take the conversion pipe).
+                        if (kVol && pending < 0 && ifirst <= ilast) {
+                            double position, p[3];
+                            point_at(ifirst, position, p);
+                            pending = (interior_axis64(p[2]).lower * dims.ny + interior_axis64(p[1]).lower) * dims.nx +
+                                      interior_axis64(p[0]).lower;
+                        }
+                        double sample = (double)ifirst + 0.5;
+                        float corners[8];
+                        int held = -1;
+#pragma unroll
+                        for (int c = 0; c < 8; ++c) corners[c] = 0.0f;
+                        for (int i = ifirst; i <= ilast; ++i) {
+                            const double position = fma(sample, step, iv.lower);
+                            const Axis64 X = interior_axis64(fma(position, r.direction[0], r.origin[0]));
+                            const Axis64 Y = interior_axis64(fma(position, r.direction[1], r.origin[1]));
+                            const Axis64 Z = interior_axis64(fma(position, r.direction[2], r.origin[2]));
+                            const int cell = (Z.lower * dims.ny + Y.lower) * dims.nx + X.lower;
+                            const double fx = X.fraction, fy = Y.fraction, fz = Z.fraction;
+                            if (kPose) {
+                                const double alpha = power_of_two ? sample * inverse_samples : sample / (double)S;
+                                f.refresh(cell, held, X.lower, Y.lower, Z.lower, corners);
+                                held = cell;
+                                double v[8], gs[3];
+#pragma unroll
+                                for (int c = 0; c < 8; ++c) v[c] = (double)corners[c];
+                                mean = mean + interpolate64(fx, fy, fz, v);
+                                interior_slope64(fx, fy, fz, v, gs);
+#pragma unroll
+                                for (int k = 0; k < 3; ++k) {
+                                    dO[k] = dO[k] + gs[k];
+                                    dD[k] = fma(position, gs[k], dD[k]);
+                                }
+                                const double along =
+                                    fma(gs[2], r.direction[2], fma(gs[1], r.direction[1], gs[0] * r.direction[0]));
+                                sl = fma(1.0 - alpha, along, sl);
+                                su = fma(alpha, along, su);
+                            }
+                            if (kVol) {
+                                red_add_run(acc, pending, cell, cs);
+                                const float keep = cell == pending ? 1.0f : 0.0f;
+                                pending = cell;
+                                const double px = vf * fx, qx = vf * (1.0 - fx), ay = 1.0 - fy, az = 1.0 - fz;
+                                const double plane[4] = {qx * ay, px * ay, qx * fy, px * fy};
+#pragma unroll
+                                for (int c = 0; c < 8; ++c)
+                                    cs[c] = fmaf(cs[c], keep, (float)(plane[c & 3] * ((c & 4) ? fz : az)));
+                            }
+                            sample = sample + 1.0;
+                        }
+                        for (int i = max(ilast + 1, split); i <= last; ++i) visit(i, true);
+                        trailing_zero = last < S - 1;
                     }
                     if (kVol && pending >= 0) flush64();
-                    if (kPose) {
+                    if constexpr (kMoments == kStoreMoments) {
+                        // the forward image, as the forward kernel forms it
+                        const double total = (trailing_zero ? mean + 0.0 : mean) * (r.length * step);
+                        if (!isfinite(total)) bits |= 2;
+                        stored_image = total;
+                        stored[0] = mean;
+#pragma unroll
+                        for (int k = 0; k < 3; ++k) {
+                            stored[1 + k] = dO[k];
+                            stored[4 + k] = dD[k];
+                        }
+                        stored[7] = sl;
+                        stored[8] = su;
+                    } else if (kPose) {
                         double lo_o[3], lo_d[3], up_o[3], up_d[3];
                         iv.lower_gradients(lo_o, lo_d);
                         iv.upper_gradients(up_o, up_d);
@@ -942,7 +1040,7 @@ __global__ void __launch_bounds__(kVjpBlock, vjp_min_blocks<kArith, kVol, kPose,
                     float words[kMomentWords] = {};
                     if constexpr (kMoments == kLoadMoments) {
 #pragma unroll
-                        for (int k = 0; k < kMomentWords; ++k) words[k] = ma.moments[k * ma.stride + ray_index];
+                        for (int k = 0; k < kMomentWords; ++k) words[k] = static_cast<const float*>(ma.moments)[k * ma.stride + ray_index];
                     } else if (segment_form(entry, sv)) {
                         // segment form: every cell run in closed form
                         int first, last;
@@ -1135,9 +1233,10 @@ __global__ void __launch_bounds__(kVjpBlock, vjp_min_blocks<kArith, kVol, kPose,
     if constexpr (kMoments == kStoreMoments) {
         if (active) {
             const int64_t ray_index = view_local * rays_per_view + pixel;
-            ma.image[ray_index] = stored_image;
+            static_cast<Word*>(ma.image)[ray_index] = stored_image;
+            Word* words = static_cast<Word*>(ma.moments) + ray_index;
 #pragma unroll
-            for (int k = 0; k < kMomentWords; ++k) ma.moments[k * ma.stride + ray_index] = stored[k];
+            for (int k = 0; k < kMomentWords; ++k) words[k * ma.stride] = stored[k];
         }
         if (bits) atomicOr(a.status + view, bits);
         return;
@@ -1242,10 +1341,10 @@ cudaError_t launch_vjp(const dpt_problem& p, const RayArgs& a, const void* packe
     return run(QuadF32{static_cast<const float4*>(packed), p.nx, p.ny, p.nz});
 }
 
-// Forward image plus the pose moments of every ray (FP32 or compensated arithmetic; see
-// kStoreMoments).
+// Forward image plus the pose moments of every ray (FP32, compensated or strict FP64
+// arithmetic; see kStoreMoments).
 cudaError_t launch_forward_moments(const dpt_problem& p, const RayArgs& a, const void* packed,
-                                   float* image, float* moments, int64_t stride, cudaStream_t stream)
+                                   void* image, void* moments, int64_t stride, cudaStream_t stream)
 {
     const dim3 grid(ray_blocks(a));
     const MomentArgs ma{moments, stride, image};
@@ -1260,17 +1359,23 @@ cudaError_t launch_forward_moments(const dpt_problem& p, const RayArgs& a, const
                 return;
             }
         }
-        k_vjp<kArith, FieldT, false, true, float, kStoreMoments>
+        k_vjp<kArith, FieldT, false, true, MomentWord<kArith>, kStoreMoments>
             <<<grid, kVjpBlock, 0, stream>>>(a, f, nullptr, 6, nullptr, nullptr, ma);
     };
     using F32 = std::integral_constant<int, DPT_ARITH_F32>;
     using F32C = std::integral_constant<int, DPT_ARITH_F32C>;
+    using F64 = std::integral_constant<int, DPT_ARITH_F64>;
     const PlainF32 direct{static_cast<const float*>(packed), p.nx, p.ny, p.nz};
     if (p.arith == DPT_ARITH_F32C) {
         if (p.layout == DPT_LAYOUT_DIRECT)
             run(F32C{}, direct);
         else
             run(F32C{}, PolyF32{static_cast<const float4*>(packed), p.nx, p.ny, p.nz});
+    } else if (p.arith == DPT_ARITH_F64) {
+        if (p.layout == DPT_LAYOUT_DIRECT)
+            run(F64{}, direct);
+        else
+            run(F64{}, QuadF32{static_cast<const float4*>(packed), p.nx, p.ny, p.nz});
     } else if (p.layout == DPT_LAYOUT_DIRECT) {
         run(F32{}, direct);
     } else {
@@ -1280,13 +1385,13 @@ cudaError_t launch_forward_moments(const dpt_problem& p, const RayArgs& a, const
 }
 
 // Pose VJP from stored moments: no sampling, the field is not read.
-cudaError_t launch_pose_from_moments(const dpt_problem& p, const RayArgs& a, const float* moments,
+cudaError_t launch_pose_from_moments(const dpt_problem& p, const RayArgs& a, const void* moments,
                                      int64_t stride, const void* cotangent, int flags,
                                      double* partials, cudaStream_t stream)
 {
     const dim3 grid(ray_blocks(a));
     const int mode = (flags & DPT_VJP_POSE12) ? 12 : ((flags & DPT_VJP_PER_RAY6) ? -6 : 6);
-    const MomentArgs ma{const_cast<float*>(moments), stride, nullptr};
+    const MomentArgs ma{const_cast<void*>(moments), stride, nullptr};
     const PlainF32 none{nullptr, p.nx, p.ny, p.nz};
     auto run = [&](auto arith, const auto* seed) {
         using SeedT = std::remove_cv_t<std::remove_pointer_t<decltype(seed)>>;
@@ -1295,7 +1400,9 @@ cudaError_t launch_pose_from_moments(const dpt_problem& p, const RayArgs& a, con
     };
     using F32 = std::integral_constant<int, DPT_ARITH_F32>;
     using F32C = std::integral_constant<int, DPT_ARITH_F32C>;
-    if (p.image_dtype == DPT_F64) {
+    if (p.arith == DPT_ARITH_F64) {
+        run(std::integral_constant<int, DPT_ARITH_F64>{}, static_cast<const double*>(cotangent));
+    } else if (p.image_dtype == DPT_F64) {
         const double* seed = static_cast<const double*>(cotangent);
         if (p.arith == DPT_ARITH_F32C) run(F32C{}, seed); else run(F32{}, seed);
     } else {

@@ -447,11 +447,19 @@ class ProjectionWorkspace:
     # Largest stored pose moments (FP32 words) a workspace keeps between a forward and its VJP.
     MOMENT_BYTES_LIMIT = 16 << 30
 
+    def _moment_bytes(self) -> int:
+        """Bytes of this workspace's stored pose moments (FP32 words, FP64 for strict FP64)."""
+        lib = N.library()
+        query = lib.dpt_b200_moments64_bytes if self.spec.arith == N.ARITH_F64 else lib.dpt_b200_moments_bytes
+        return query(self.problem, self.views)
+
     def moments_supported(self) -> bool:
         """Whether a forward can store the pose moments for a later pose VJP (FP32 or
-        compensated arithmetic, FP32 images, within MOMENT_BYTES_LIMIT)."""
-        return (self.spec.arith in (N.ARITH_F32, N.ARITH_F32C) and self.spec.image_code == N.F32 and
-                N.library().dpt_b200_moments_bytes(self.problem, self.views) <= self.MOMENT_BYTES_LIMIT)
+        compensated arithmetic with FP32 images, strict FP64 with FP64 images, within
+        MOMENT_BYTES_LIMIT)."""
+        forms = ((N.ARITH_F32, N.F32), (N.ARITH_F32C, N.F32), (N.ARITH_F64, N.F64))
+        return ((self.spec.arith, self.spec.image_code) in forms
+                and self._moment_bytes() <= self.MOMENT_BYTES_LIMIT)
 
     def moments_preferred(self) -> bool:
         """Whether a training step should store the pose moments in its forward (and run the
@@ -459,8 +467,26 @@ class ProjectionWorkspace:
         pose VJP.  Measured on 64 views of the 256^3 / 512^2 / S = 1024 full scan: FP32
         arithmetic 101.1 ms split against 114.5 ms joint; the compensated form 65.4 ms split
         against 64.2 ms joint (its moment-storing forward costs more than the pose terms add
-        to a pass bound by its scatter)."""
-        return self.spec.arith == N.ARITH_F32 and self.moments_supported()
+        to a pass bound by its scatter).  Strict FP64, 16 views:
+        forward and VJP 39 ms split, 51 ms joint."""
+        return self.spec.arith in (N.ARITH_F32, N.ARITH_F64) and self.moments_supported()
+
+    def _allocate_moments(self) -> bool:
+        """Hold storage for the pose moments; False where they are not supported, or the strict
+        FP64 ones (twice the words of FP32) do not fit the device beside the caller's tensors."""
+        if not self.moments_supported():
+            return False
+        size = self._moment_bytes()
+        wide = self.spec.arith == N.ARITH_F64
+        if self._moments is None or self._moments.numel() * self._moments.element_size() < size:
+            try:
+                self._moments = torch.empty(size // (8 if wide else 4), device=self.device,
+                                            dtype=torch.float64 if wide else torch.float32)
+            except torch.OutOfMemoryError:
+                if not wide:
+                    raise
+                return False
+        return True
 
     def _moments_match(self, field: torch.Tensor, poses: torch.Tensor) -> bool:
         """Whether the stored moments belong to these inputs.  The workspace holds the
@@ -477,7 +503,7 @@ class ProjectionWorkspace:
                 *, checked: bool = True, moments: bool = False) -> torch.Tensor:
         """Optical depth ``(views, rows, cols)`` (bundles: ``(rays,)``).
 
-        ``moments=True`` (FP32 or compensated arithmetic) also stores each ray's pose moments, so that a
+        ``moments=True`` (FP32, compensated or strict FP64 arithmetic) also stores each ray's pose moments, so that a
         following ``vjp`` with the same field and poses forms the pose gradient without
         sampling again; the image is identical either way."""
         with self.lock, torch.cuda.device(self.device):
@@ -490,12 +516,11 @@ class ProjectionWorkspace:
                 raise ContractError("out must match the projector's shape, dtype and input device")
             packed = self.prepare_field(field, poses)
             self._moments_for = None
-            if moments and self.moments_supported():
+            if moments and self._allocate_moments():
                 lib = N.library()
-                size = lib.dpt_b200_moments_bytes(self.problem, self.views)
-                if self._moments is None or self._moments.numel() * 4 < size:
-                    self._moments = torch.empty(size // 4, dtype=torch.float32, device=self.device)
-                self._run("forward_moments", lambda: lib.dpt_b200_forward_moments(
+                call = (lib.dpt_b200_forward_moments64 if self.spec.arith == N.ARITH_F64
+                        else lib.dpt_b200_forward_moments)
+                self._run("forward_moments", lambda: call(
                     self.problem, self.rays(poses), packed.data_ptr(), out.data_ptr(),
                     self._moments.data_ptr(), self.status.data_ptr(), _stream(self.device)))
                 self._moments_for = (field, poses, field._version, poses._version)
@@ -547,7 +572,9 @@ class ProjectionWorkspace:
             # launch-log label: what each sampling launch computes
             label = "vjp" if (volume and components and not split) else "vjp_volume" if volume else "vjp_pose"
             if split:
-                self._run("pose_from_moments", lambda: lib.dpt_b200_pose_from_moments(
+                form = (lib.dpt_b200_pose_from_moments64 if self.spec.arith == N.ARITH_F64
+                        else lib.dpt_b200_pose_from_moments)
+                self._run("pose_from_moments", lambda: form(
                     self.problem, self.rays(poses), self._moments.data_ptr(), cot.data_ptr(),
                     N.VJP_POSE12 if components == 12 else N.VJP_POSE6, partials.data_ptr(),
                     self.status.data_ptr(), stream))

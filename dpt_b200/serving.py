@@ -813,7 +813,8 @@ class ProjectionServer:
         """Launch sequence of one request on the current stream (no host synchronisation).
         A pose request in FP32 arithmetic stores its rays' pose moments in the forward, so its
         pose VJP applies the residual without a second sampling pass."""
-        moments = request.kind == "pose" and ws.moments_preferred()
+        # (strict FP64 moments are not in request_bytes: its pose requests sample again)
+        moments = request.kind == "pose" and request.precision != "fp64" and ws.moments_preferred()
         image = ws.forward(field_tensor, inputs["poses"], checked=False, moments=moments)
         out = {"image": image}
         if request.kind != "forward":

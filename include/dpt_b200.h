@@ -242,6 +242,15 @@ int dpt_b200_pose_from_moments(const dpt_problem* problem, const dpt_rays* rays,
                                const void* cotangent, int32_t flags, double* pose_partials,
                                int32_t* status, void* stream);
 
+/* The same for the strict FP64 arithmetic (DPT_ARITH_F64, FP64 images): nine FP64 words per
+ * ray. */
+size_t dpt_b200_moments64_bytes(const dpt_problem* problem, int32_t view_count);
+int dpt_b200_forward_moments64(const dpt_problem* problem, const dpt_rays* rays, const void* packed,
+                               double* image, double* moments, int32_t* status, void* stream);
+int dpt_b200_pose_from_moments64(const dpt_problem* problem, const dpt_rays* rays, const double* moments,
+                                 const double* cotangent, int32_t flags, double* pose_partials,
+                                 int32_t* status, void* stream);
+
 /* Reduce the pose partials of a dpt_b200_vjp call over views [view_begin, view_begin +
  * view_count) in a fixed FP64 order into `pose_gradient` (view_count x components,
  * components 12 or 6); accumulate != 0 adds.  Non-finite results set bit 2 of
