@@ -52,6 +52,7 @@ EXPORTS = (
     "dpt_b200_moments64_bytes",
     "dpt_b200_forward_moments64",
     "dpt_b200_pose_from_moments64",
+    "dpt_b200_pose_chart_vjp",
     "dpt_b200_gather_plan_bytes",
     "dpt_b200_gather_prepare",
     "dpt_b200_gather_count",
@@ -134,6 +135,7 @@ _SIGNATURES = {
     "dpt_b200_moments64_bytes": ([_P, _I], ctypes.c_size_t),
     "dpt_b200_forward_moments64": ([_P, _R, _V, _V, _V, _V, _V], ctypes.c_int),
     "dpt_b200_pose_from_moments64": ([_P, _R, _V, _V, _I, _V, _V, _V], ctypes.c_int),
+    "dpt_b200_pose_chart_vjp": ([_I, _V, _V, _V, _V, _V], ctypes.c_int),
     "dpt_b200_gather_plan_bytes": ([_P, _I], ctypes.c_size_t),
     "dpt_b200_gather_prepare": ([_P, _R, _V, _V, _V], ctypes.c_int),
     "dpt_b200_gather_count": ([_P, _R, _V, _I, _V, _V], ctypes.c_int),

@@ -43,6 +43,8 @@ cudaError_t launch_pose_from_moments(const dpt_problem& p, const RayArgs& a, con
 cudaError_t launch_finish_pose(int view_begin, int view_count, int tiles, int components,
                                const double* partials, double* gradient, int accumulate,
                                int32_t* status, cudaStream_t stream);
+cudaError_t launch_chart_vjp(int views, const double* poses, const double* tangents, const double* cotangents,
+                             double* gradients, cudaStream_t stream);
 cudaError_t launch_fold(const dpt_problem& p, float* accumulator, double* total,
                         int accumulate_total, void* gradient, int gradient_dtype, int clear,
                         int32_t* status, cudaStream_t stream);

@@ -32,11 +32,13 @@ from threading import RLock
 
 import torch
 
+from .. import _native as N
 from ..contracts import ContractError, integer
 from ..geometry import BatchedGeometry, CurvedDetectorGeometry, DetectorGeometry, ParallelGeometry
 from ..projection import ProjectionSpec, ProjectionWorkspace
 from ..plan import plan_rays
 from ..volumes import GridSpec
+from .geometry import compose_pose
 
 _CACHE_LIMIT = 8
 _CACHE: OrderedDict[tuple, ProjectionWorkspace] = OrderedDict()
@@ -270,3 +272,54 @@ def _out_fake(field, poses, value, out):
     shape, dtype = metadata(field, poses, value)
     if tuple(out.shape) != shape or out.dtype != dtype or out.device != field.device or not out.is_contiguous():
         raise ContractError("out must match the projector's shape, dtype and input device")
+
+
+# ------------------------------------------------------------ poses about a fixed anchor
+
+@torch.library.custom_op("dpt::compose_pose", mutates_args=())
+def compose_fixed_anchor(anchor: torch.Tensor, tangent: torch.Tensor) -> torch.Tensor:
+    """``compose_pose`` of CUDA tensors, an anchor without gradient and a tangent per pose: the
+    same poses, with the tangents' first-order gradient from one kernel (the reverse pass of
+    ``matrix_exp`` takes some 90 launches, 0.9 ms of a two-view registration step).  (One tangent
+    for a row of anchors keeps Torch's reverse pass: ``matmul`` folds that product, and so rounds
+    it, differently when it records a gradient.)"""
+    return compose_pose(anchor, tangent)
+
+
+@compose_fixed_anchor.register_fake
+def _compose_fake(anchor, tangent):
+    leading = torch.broadcast_shapes(anchor.shape[:-1], tangent.shape[:-1])
+    return tangent.new_empty((*leading, 12))
+
+
+@torch.library.custom_op("dpt::compose_pose_vjp", mutates_args=())
+def compose_fixed_anchor_vjp(poses: torch.Tensor, tangent: torch.Tensor, cotangent: torch.Tensor) -> torch.Tensor:
+    """Tangent cotangent of packed ``poses`` ``(12,)`` or ``(views, 12)`` from theirs."""
+    poses, tangent, cotangent = poses.contiguous(), tangent.contiguous(), cotangent.contiguous()
+    gradient = torch.empty_like(tangent)
+    views = tangent.numel() // 6
+    if poses.numel() != 12 * views or cotangent.numel() != 12 * views:
+        raise ContractError("compose_pose_vjp needs a tangent per pose")
+    with torch.cuda.device(tangent.device):
+        stream = torch.cuda.current_stream(tangent.device).cuda_stream
+        N.check(N.library().dpt_b200_pose_chart_vjp(views, poses.data_ptr(), tangent.data_ptr(),
+                                                    cotangent.data_ptr(), gradient.data_ptr(), stream),
+                "compose_pose_vjp")
+    return gradient
+
+
+@compose_fixed_anchor_vjp.register_fake
+def _compose_vjp_fake(poses, tangent, cotangent):
+    return torch.empty_like(tangent)
+
+
+def _compose_setup(ctx, inputs, output):
+    ctx.save_for_backward(output, inputs[1])
+
+
+def _compose_backward(ctx, cotangent):
+    poses, tangent = ctx.saved_tensors
+    return None, compose_fixed_anchor_vjp(poses, tangent, cotangent)
+
+
+compose_fixed_anchor.register_autograd(_compose_backward, setup_context=_compose_setup)

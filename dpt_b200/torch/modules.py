@@ -200,7 +200,11 @@ class Projector(torch.nn.Module):
                 TANGENT.check(pose, self.views)
                 if pose.device != field.device:
                     raise ContractError("pose and field must share a device")
-                packed = compose_pose(anchor, pose)
+                if (pose.requires_grad and torch.is_grad_enabled() and not anchor.requires_grad
+                        and pose.ndim >= anchor.ndim):
+                    packed = _projection_ops.compose_fixed_anchor(anchor, pose)
+                else:
+                    packed = compose_pose(anchor, pose)
         if packed.device != field.device:
             raise ContractError("packed_pose and field must share a device")
         return packed if packed.ndim == 2 else packed.expand(self.views, 12)

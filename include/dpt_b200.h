@@ -251,6 +251,12 @@ int dpt_b200_pose_from_moments64(const dpt_problem* problem, const dpt_rays* ray
                                  const double* cotangent, int32_t flags, double* pose_partials,
                                  int32_t* status, void* stream);
 
+/* VJP of the rigid chart pose = anchor exp(tangent^) (python/dpt/torch/geometry.py:19-63) with
+ * respect to the tangent: the composed `poses` and their `cotangents` (views x 12), the
+ * `tangents` (views x 6); writes `gradients` (views x 6). */
+int dpt_b200_pose_chart_vjp(int32_t views, const double* poses, const double* tangents,
+                            const double* cotangents, double* gradients, void* stream);
+
 /* Reduce the pose partials of a dpt_b200_vjp call over views [view_begin, view_begin +
  * view_count) in a fixed FP64 order into `pose_gradient` (view_count x components,
  * components 12 or 6); accumulate != 0 adds.  Non-finite results set bit 2 of
