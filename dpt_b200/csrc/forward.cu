@@ -23,14 +23,16 @@
 #include "launch.h"
 
 // Resident blocks per SM the register allocation must allow.  FP32: 32 views of the 256^3 /
-// 512^2 / S = 1024 scan take 12.4 ms at eight blocks (62 registers), 12.8 at nine (56).
+// 512^2 / S = 1024 scan take 12.3 ms at six blocks (69 registers), 12.5 at eight (64), 12.8 at
+// nine (56).
 #ifndef DPT_FORWARD_MIN_BLOCKS_F32
-#define DPT_FORWARD_MIN_BLOCKS_F32 8
+#define DPT_FORWARD_MIN_BLOCKS_F32 6
 #endif
-// Strict FP64: 16 views take 10.8 ms at seven blocks (72 registers, 36 bytes spilled), 11.0 at
-// six (80 registers, two samples unrolled).
+// Strict FP64: 16 views of that scan 10.3 ms at five blocks (94 registers), 10.2 at six, 9.9 at
+// seven (72); launches of a few waves and less gain more from the registers (8 views of 64^2 of a
+// 64^3 volume 46, 60 and 56 us, 16 views of 117 x 145 at S = 336 170, 200 and 216 us).
 #ifndef DPT_FORWARD_MIN_BLOCKS_F64
-#define DPT_FORWARD_MIN_BLOCKS_F64 7
+#define DPT_FORWARD_MIN_BLOCKS_F64 5
 #endif
 
 namespace dpt {
@@ -134,8 +136,11 @@ __device__ __forceinline__ void forward_tile(const RayArgs& a, const Field& f, O
                         at(i, x, y, z);
                         return inside(x, y, z, dims.hx, dims.hy, dims.hz);
                     }, first, last);
+                    // the pairs' floors need coordinates, and the exact sample parameters
+                    // i + 0.5, below 2^23
+                    const bool pairs = dims.packed && S <= (1 << 23);
                     int ifirst, ilast;
-                    interior_run(first, last, [&](int i) {
+                    const bool separate = short_margins(first, last, [&](int i) {
                         float x, y, z;
                         at(i, x, y, z);
                         return x >= 0.0f && x < dims.mx && y >= 0.0f && y < dims.my && z >= 0.0f && z < dims.mz;
@@ -152,30 +157,32 @@ __device__ __forceinline__ void forward_tile(const RayArgs& a, const Field& f, O
                         at(i, x, y, z);
                         add(axis32(x, dims.mx, dims.cx), axis32(y, dims.my, dims.cy), axis32(z, dims.mz, dims.cz));
                     };
-                    const int split = min(ifirst, last + 1);
-                    for (int i = first; i < split; ++i) margin(i);
-                    int i = ifirst;
-                    // Samples i and i + 1 of the interior run at once: positions, floors and corner
+                    // Samples i and i + 1 at once up to `end`: positions, floors and corner
                     // weights lane-wise (see "packed FP32 pairs" in common.cuh), the corners
                     // reloaded under a predicate, the ray sum serial in sample order, so the total
                     // is the one the scalar samples form.  The kernel is bound by issue slots: 32
                     // views of the 256^3 / 512^2 / S = 1024 scan 13.9 -> 12.4 ms (54 -> 44 thread
-                    // instructions per sample).  The floors need coordinates, and the exact
-                    // sample parameters i + 0.5, below 2^23.
-                    if (dims.packed && S <= (1 << 23)) {
+                    // instructions per sample).  Returns the first sample left.
+                    auto march = [&](int i, int end, auto clamped) {
                         f32x2 ip = pack2((float)i + 0.5f, (float)i + 1.5f);
                         BiasedCells cells;
                         cells.init(dims.nx, dims.ny);
-                        for (; i + 1 <= ilast; i += 2) {
+                        for (; i + 1 <= end; i += 2) {
                             const f32x2 position = fma2(ip, splat2(step), splat2(iv.lower));
                             ip = add2(ip, splat2(2.0f));
                             const f32x2 x = fma2(position, splat2(d[0]), splat2(o[0]));
                             const f32x2 y = fma2(position, splat2(d[1]), splat2(o[1]));
                             const f32x2 z = fma2(position, splat2(d[2]), splat2(o[2]));
-                            f32x2 bx, by, bz;
-                            const f32x2 fx = interior_fraction2(x, &bx);
-                            const f32x2 fy = interior_fraction2(y, &by);
-                            const f32x2 fz = interior_fraction2(z, &bz);
+                            f32x2 bx, by, bz, fx, fy, fz;
+                            if constexpr (decltype(clamped)::value) {
+                                fx = capped_fraction2(clamp2(x, dims.mx), dims.cx, &bx);
+                                fy = capped_fraction2(clamp2(y, dims.my), dims.cy, &by);
+                                fz = capped_fraction2(clamp2(z, dims.mz), dims.cz, &bz);
+                            } else {
+                                fx = interior_fraction2(x, &bx);
+                                fy = interior_fraction2(y, &by);
+                                fz = interior_fraction2(z, &bz);
+                            }
                             f32x2 w[8];
                             corner_weights2(fx, fy, fz, w);
                             float w0[8], w1[8];
@@ -194,13 +201,18 @@ __device__ __forceinline__ void forward_tile(const RayArgs& a, const Field& f, O
                             total = total + interpolate(w1, cache.v);
                             cache.cell = cell1;
                         }
+                        return i;
+                    };
+                    if (any_in_warp(!separate)) {
+                        int i = pairs ? march(first, last, std::true_type{}) : first;
+                        for (; i <= last; ++i) margin(i);
+                    } else {
+                        const int split = min(ifirst, last + 1);
+                        for (int i = first; i < split; ++i) margin(i);
+                        int i = pairs ? march(ifirst, ilast, std::false_type{}) : ifirst;
+                        for (; i <= ilast; ++i) margin(i);
+                        for (i = max(ilast + 1, split); i <= last; ++i) margin(i);
                     }
-                    for (; i <= ilast; ++i) {
-                        float x, y, z;
-                        at(i, x, y, z);
-                        add(interior_axis(x), interior_axis(y), interior_axis(z));
-                    }
-                    for (int i = max(ilast + 1, split); i <= last; ++i) margin(i);
                     // the zero samples after the run: adding +0 only turns -0 into +0
                     if (last < S - 1) total = total + 0.0f;
                 }
@@ -372,47 +384,56 @@ __device__ __forceinline__ void forward_tile(const RayArgs& a, const Field& f, O
                     const double mx = (double)(a.grid.nx - 1), my = (double)(a.grid.ny - 1), mz = (double)(a.grid.nz - 1);
                     const int cx = max(a.grid.nx - 2, 0), cy = max(a.grid.ny - 2, 0), cz = max(a.grid.nz - 2, 0);
                     int ifirst, ilast;
-                    interior_run(first, last, [&](int i) {
+                    const bool separate = short_margins(first, last, [&](int i) {
                         double p[3];
                         at(i, p);
                         return p[0] >= 0.0 && p[0] < mx && p[1] >= 0.0 && p[1] < my && p[2] >= 0.0 && p[2] < mz;
                     }, ifirst, ilast);
-                    WideCellCache<Field> cache;
-                    auto margin = [&](int i) {
-                        double p[3];
-                        at(i, p);
-                        const Axis64 X = axis64(p[0], mx, cx), Y = axis64(p[1], my, cy), Z = axis64(p[2], mz, cz);
-                        cache.fetch(f, X.lower, Y.lower, Z.lower, (Z.lower * a.grid.ny + Y.lower) * a.grid.nx + X.lower);
-                        integral = integral + interpolate64(X.fraction, Y.fraction, Z.fraction, cache.v);
-                    };
-                    const int split = min(ifirst, last + 1);
-                    for (int i = first; i < split; ++i) margin(i);
-                    // Interior samples: no clamp, no conversion of a coordinate (interior_axis64) and
-                    // the corners reloaded under a predicate; eight widenings of the FP32 corners
-                    // stay on the conversion pipe, beside 32 FP64 operations.  16 views of the
-                    // 256^3 / 512^2 / S = 1024 scan: 14.1 -> 10.8 ms.  (FP64 corner quads of 32
-                    // bytes save those too, 10.4 ms, but a volume of 36 M voxels then waits on
-                    // L2: 3.45 against 2.80 ms for three views.)
-                    double sample = (double)ifirst + 0.5;
+                    // No conversion of a coordinate (interior_axis64) and the corners reloaded
+                    // under a predicate; eight widenings of the FP32 corners stay on the
+                    // conversion pipe, beside 32 FP64 operations.  16 views of the 256^3 / 512^2 /
+                    // S = 1024 scan: 14.1 -> 10.3 ms.  (FP64 corner quads of 32 bytes save those
+                    // too, 10.4 ms, but a volume of 36 M voxels then waits on L2: 3.45 against
+                    // 2.80 ms for three views.)
                     float corners[8];
                     int held = -1;
 #pragma unroll
                     for (int c = 0; c < 8; ++c) corners[c] = 0.0f;
-                    for (int i = ifirst; i <= ilast; ++i) {
-                        const double position = fma(sample, step, iv.lower);
-                        sample = sample + 1.0;
-                        const Axis64 X = interior_axis64(fma(position, r.direction[0], r.origin[0]));
-                        const Axis64 Y = interior_axis64(fma(position, r.direction[1], r.origin[1]));
-                        const Axis64 Z = interior_axis64(fma(position, r.direction[2], r.origin[2]));
-                        const int cell = (Z.lower * a.grid.ny + Y.lower) * a.grid.nx + X.lower;
-                        f.refresh(cell, held, X.lower, Y.lower, Z.lower, corners);
-                        held = cell;
-                        double v[8];
+                    auto march = [&](int i, int end, auto clamped) {
+                        double sample = (double)i + 0.5;
+                        for (; i <= end; ++i) {
+                            const double position = fma(sample, step, iv.lower);
+                            sample = sample + 1.0;
+                            double p[3];
 #pragma unroll
-                        for (int c = 0; c < 8; ++c) v[c] = (double)corners[c];
-                        integral = integral + interpolate64(X.fraction, Y.fraction, Z.fraction, v);
+                            for (int k = 0; k < 3; ++k) p[k] = fma(position, r.direction[k], r.origin[k]);
+                            Axis64 X, Y, Z;
+                            if constexpr (decltype(clamped)::value) {
+                                X = clamped_axis64(p[0], mx, cx);
+                                Y = clamped_axis64(p[1], my, cy);
+                                Z = clamped_axis64(p[2], mz, cz);
+                            } else {
+                                X = interior_axis64(p[0]);
+                                Y = interior_axis64(p[1]);
+                                Z = interior_axis64(p[2]);
+                            }
+                            const int cell = (Z.lower * a.grid.ny + Y.lower) * a.grid.nx + X.lower;
+                            f.refresh(cell, held, X.lower, Y.lower, Z.lower, corners);
+                            held = cell;
+                            double v[8];
+#pragma unroll
+                            for (int c = 0; c < 8; ++c) v[c] = (double)corners[c];
+                            integral = integral + interpolate64(X.fraction, Y.fraction, Z.fraction, v);
+                        }
+                    };
+                    if (any_in_warp(!separate)) {
+                        march(first, last, std::true_type{});
+                    } else {
+                        const int split = min(ifirst, last + 1);
+                        march(first, split - 1, std::true_type{});
+                        march(ifirst, ilast, std::false_type{});
+                        march(max(ilast + 1, split), last, std::true_type{});
                     }
-                    for (int i = max(ilast + 1, split); i <= last; ++i) margin(i);
                     if (last < S - 1) integral = integral + 0.0;
                 }
                 integral = integral * (r.length * step);

@@ -25,15 +25,16 @@
 #define DPT_VJP_REUSE 0
 #endif
 // Resident blocks per SM the register allocation must allow, per arithmetic (128-thread
-// blocks).  The kernels are latency bound, so occupancy pays for a few spilled registers:
-// the compensated form's cell walk measured 0.71 ms per 512^2 view (S = 1024) at four
-// blocks (118 registers), 0.59 at eight (64 registers, 376 bytes spilled to L1); the FP32
-// form 1.17 ms at five blocks (96 registers), 1.15 at six (80 registers, 12 bytes spilled).
+// blocks).  The compensated form's cell walk measured 0.71 ms per 512^2 view (S = 1024) at four
+// blocks (118 registers), 0.59 at eight (64 registers, 376 bytes spilled to L1).  The FP32
+// joint pass, without spills at four blocks (126 registers), takes 32.8 ms per 32 views of the
+// 256^3 scan, 33.0 at five and 39.9 at six (80 registers, 592 bytes spilled); 51.2 before the
+// branches left its loops.
 #ifndef DPT_VJP_MIN_BLOCKS_F32
-#define DPT_VJP_MIN_BLOCKS_F32 6
+#define DPT_VJP_MIN_BLOCKS_F32 4
 #endif
-// The FP32 volume scatter alone (per 32 views of the full scan): 16.2 ms at six blocks (80
-// registers), 16.3 at eight (64).
+// The FP32 volume scatter alone (per 32 views of the full scan): 15.5 ms at five and six blocks
+// (80 registers at six), 15.6 at eight (64).
 #ifndef DPT_VJP_MIN_BLOCKS_F32_VOLUME
 #define DPT_VJP_MIN_BLOCKS_F32_VOLUME 6
 #endif
@@ -55,21 +56,20 @@
 #ifndef DPT_VJP_MIN_BLOCKS_F32C_JOINT
 #define DPT_VJP_MIN_BLOCKS_F32C_JOINT 8
 #endif
-// The FP32 forward that stores the pose moments (per 32 views of the full scan): 24.1 ms at
-// four and five blocks (none spilled), 25.0 at six (80 registers, 76 bytes spilled), 25.8 at
-// seven; the occupancy does not matter where the FP32 pipe binds.
+// The FP32 forward that stores the pose moments (per 32 views of the full scan): 23.9 ms at
+// four blocks, 23.6 at five, and with more spilled 25.0 at six (80 registers), 25.8 at seven.
 #ifndef DPT_VJP_MIN_BLOCKS_F32_MOMENTS
 #define DPT_VJP_MIN_BLOCKS_F32_MOMENTS 5
 #endif
-// Strict FP64, 16 views of the full scan: the pose pass 23.0 ms at four blocks (128 registers,
-// 212 bytes spilled), 25.1 at five (96, 452 bytes); the volume scatter 15.2 ms at six blocks
-// (80 registers), 15.8 at seven (72).  The cell-Gauss joint VJP: 61.5 ms per 32 views at three
-// blocks, 59.3 at four, 66.0 at five.  The mixed and fast forms keep three.
+// Strict FP64, 16 views of the full scan: the forward that stores the moments 19.4 ms at three
+// blocks (126 registers), 19.9 at four (120), 21.1 at five (96); the volume scatter 11.3 ms at
+// five blocks (96 registers), 11.6 at six and eight.  The cell-Gauss joint VJP: 61.5 ms per 32
+// views at three blocks, 59.3 at four, 66.0 at five.  The mixed and fast forms keep three.
 #ifndef DPT_VJP_MIN_BLOCKS_F64
-#define DPT_VJP_MIN_BLOCKS_F64 4
+#define DPT_VJP_MIN_BLOCKS_F64 3
 #endif
 #ifndef DPT_VJP_MIN_BLOCKS_F64_VOLUME
-#define DPT_VJP_MIN_BLOCKS_F64_VOLUME 6
+#define DPT_VJP_MIN_BLOCKS_F64_VOLUME 5
 #endif
 #ifndef DPT_VJP_MIN_BLOCKS_CELLS
 #define DPT_VJP_MIN_BLOCKS_CELLS 4
@@ -259,8 +259,7 @@ __global__ void __launch_bounds__(kVjpBlock, vjp_min_blocks<kArith, kVol, kPose,
                     int held = -1;  // the cell of the pair loop's corners
                     const float inverse_samples = 1.0f / (float)S;
                     // One midpoint.  mode 0: general (support and finiteness tested); 1: on the
-                    // inside run (both known to pass); 2: on the interior run (no clamp active,
-                    // slope masks 1).
+                    // inside run (both known to pass).
                     // `bounded` (every increment finite and at most 1 in magnitude) is fixed
                     // per ray: the march is instantiated for both values so the sample loop
                     // carries no test of it
@@ -279,11 +278,7 @@ __global__ void __launch_bounds__(kVjpBlock, vjp_min_blocks<kArith, kVol, kPose,
                         Axis32 X{0, 0.0f}, Y{0, 0.0f}, Z{0, 0.0f};
                         float w[8];
                         int cell = -1;
-                        if (mode == 2) {
-                            X = interior_axis(x);
-                            Y = interior_axis(y);
-                            Z = interior_axis(z);
-                        } else if (in) {
+                        if (in) {
                             X = axis32(x, dims.mx, dims.cx);
                             Y = axis32(y, dims.my, dims.cy);
                             Z = axis32(z, dims.mz, dims.cz);
@@ -297,10 +292,9 @@ __global__ void __launch_bounds__(kVjpBlock, vjp_min_blocks<kArith, kVol, kPose,
                             if (in) {
                                 cache.fetch(f, X.lower, Y.lower, Z.lower, cell);
                                 value = interpolate(w, cache.v);
-                                const bool core = mode == 2;
-                                const float sx = (core || (x >= 0.0f && x < dims.mx)) ? 1.0f : 0.0f;
-                                const float sy = (core || (y >= 0.0f && y < dims.my)) ? 1.0f : 0.0f;
-                                const float sz = (core || (z >= 0.0f && z < dims.mz)) ? 1.0f : 0.0f;
+                                const float sx = (x >= 0.0f && x < dims.mx) ? 1.0f : 0.0f;
+                                const float sy = (y >= 0.0f && y < dims.my) ? 1.0f : 0.0f;
+                                const float sz = (z >= 0.0f && z < dims.mz) ? 1.0f : 0.0f;
                                 slope32(X.fraction, Y.fraction, Z.fraction, cache.v, sx, sy, sz, gs);
                             }
                             mean = mean + value;
@@ -371,26 +365,33 @@ __global__ void __launch_bounds__(kVjpBlock, vjp_min_blocks<kArith, kVol, kPose,
                             }
                         }
                     };
-                    // Samples i and i + 1 of the interior run, lane-wise where the arithmetic is
+                    // Samples i and i + 1 of the interior run (with kClamped: of the inside run,
+                    // whose clamps and slope masks then apply), lane-wise where the arithmetic is
                     // (see "packed FP32 pairs" in common.cuh); the serial sums take sample i,
                     // then sample i + 1, so every moment, increment and run sum is the value
-                    // the two visits of mode 2 form.  `ip` holds (i + 0.5, i + 1.5).  Positions and
+                    // the two visits form.  `ip` holds (i + 0.5, i + 1.5).  Positions and
                     // coordinates stay scalar (a packed operand of a per-ray value takes two
                     // registers).  The corners reload, and a finished run flushes, under a
                     // predicate instead of a branch: 32 views of the 256^3 / 512^2 / S = 1024
-                    // scan take 39.0 ms jointly (51.2 before), 24.1 storing the moments (25.2),
-                    // 16.2 scattering (16.3); 512^3 at 0.5 mm, 16 views: 14.4 (15.6) and 29.0 (31.3).
-                    auto visit_pair = [&](int i, f32x2 ip, auto bounded_tag, auto pow2_tag) {
-                        (void)bounded_tag;
+                    // scan take 32.8 ms jointly (51.2 before), 23.6 storing the moments (25.2),
+                    // 15.5 scattering (16.3); 512^3 at 0.5 mm, 16 views: 14.4 (15.6) and 29.0 (31.3).
+                    auto visit_pair = [&](int i, f32x2 ip, auto pow2_tag, auto clamped_tag) {
+                        constexpr bool kClamped = decltype(clamped_tag)::value;
                         const float q0 = fmaf(lo2(ip), step, iv.lower), q1 = fmaf(hi2(ip), step, iv.lower);
                         const f32x2 position = pack2(q0, q1);
                         const f32x2 x = pack2(fmaf(q0, d[0], o[0]), fmaf(q1, d[0], o[0]));
                         const f32x2 y = pack2(fmaf(q0, d[1], o[1]), fmaf(q1, d[1], o[1]));
                         const f32x2 z = pack2(fmaf(q0, d[2], o[2]), fmaf(q1, d[2], o[2]));
-                        f32x2 bx, by, bz;
-                        const f32x2 fx = interior_fraction2(x, &bx);
-                        const f32x2 fy = interior_fraction2(y, &by);
-                        const f32x2 fz = interior_fraction2(z, &bz);
+                        f32x2 bx, by, bz, fx, fy, fz;
+                        if constexpr (kClamped) {
+                            fx = capped_fraction2(clamp2(x, dims.mx), dims.cx, &bx);
+                            fy = capped_fraction2(clamp2(y, dims.my), dims.cy, &by);
+                            fz = capped_fraction2(clamp2(z, dims.mz), dims.cz, &bz);
+                        } else {
+                            fx = interior_fraction2(x, &bx);
+                            fy = interior_fraction2(y, &by);
+                            fz = interior_fraction2(z, &bz);
+                        }
                         const int lx0 = biased_lo(bx), ly0 = biased_lo(by), lz0 = biased_lo(bz);
                         const int lx1 = biased_hi(bx), ly1 = biased_hi(by), lz1 = biased_hi(bz);
                         const int cell0 = cells.at<kPow2>(lo2(bx), lo2(by), lo2(bz));
@@ -416,6 +417,11 @@ __global__ void __launch_bounds__(kVjpBlock, vjp_min_blocks<kArith, kVol, kPose,
                             held = cell1;
                             f32x2 gs[3];
                             slope2(fx, fy, fz, ax, ay, az, du, dv, gs);
+                            if constexpr (kClamped) {
+                                gs[0] = mul2(slope_mask2(x, dims.mx), gs[0]);
+                                gs[1] = mul2(slope_mask2(y, dims.my), gs[1]);
+                                gs[2] = mul2(slope_mask2(z, dims.mz), gs[2]);
+                            }
                             mean = mean + value0;
                             mean = mean + value1;
                             const float p0 = lo2(position), p1 = hi2(position);
@@ -467,33 +473,40 @@ __global__ void __launch_bounds__(kVjpBlock, vjp_min_blocks<kArith, kVol, kPose,
                                           fmaf(position, d[2], o[2]), dims.hx, dims.hy, dims.hz);
                         }, first, last);
                         int ifirst, ilast;
-                        interior_run(first, last, [&](int i) {
+                        const bool separate = short_margins(first, last, [&](int i) {
                             const float position = position_at(i);
                             const float x = fmaf(position, d[0], o[0]), y = fmaf(position, d[1], o[1]),
                                         z = fmaf(position, d[2], o[2]);
                             return x >= 0.0f && x < dims.mx && y >= 0.0f && y < dims.my && z >= 0.0f && z < dims.mz;
                         }, ifirst, ilast);
-                        const int split = min(ifirst, last + 1);
-                        for (int i = first; i < split; ++i) visit(i, 1, bounded_tag, pow2_tag);
-                        int i = ifirst;
-                        // the pair floors need interior coordinates below 2^23, and the pair
-                        // scatter bounded increments
-                        if (dims.packed && S <= (1 << 23) && (!kVol || decltype(bounded_tag)::value)) {
+                        // the pair floors need coordinates and sample parameters below 2^23, and
+                        // the pair scatter bounded increments
+                        const bool pairs = dims.packed && S <= (1 << 23) && (!kVol || decltype(bounded_tag)::value);
+                        auto march_pairs = [&](int i, int end, auto clamped_tag) {
                             f32x2 ip = pack2((float)i + 0.5f, (float)i + 1.5f);
-                            if (kVol && pending < 0 && i < ilast) {
+                            if (kVol && pending < 0 && i < end) {
                                 const float position = position_at(i);
-                                const Axis32 X = interior_axis(fmaf(position, d[0], o[0]));
-                                const Axis32 Y = interior_axis(fmaf(position, d[1], o[1]));
-                                const Axis32 Z = interior_axis(fmaf(position, d[2], o[2]));
+                                const Axis32 X = axis32(fmaf(position, d[0], o[0]), dims.mx, dims.cx);
+                                const Axis32 Y = axis32(fmaf(position, d[1], o[1]), dims.my, dims.cy);
+                                const Axis32 Z = axis32(fmaf(position, d[2], o[2]), dims.mz, dims.cz);
                                 pending = (Z.lower * dims.ny + Y.lower) * dims.nx + X.lower;
                             }
-                            for (; i + 1 <= ilast; i += 2) {
-                                visit_pair(i, ip, bounded_tag, pow2_tag);
+                            for (; i + 1 <= end; i += 2) {
+                                visit_pair(i, ip, pow2_tag, clamped_tag);
                                 ip = add2(ip, splat2(2.0f));
                             }
+                            return i;
+                        };
+                        if (any_in_warp(!separate)) {
+                            int i = pairs ? march_pairs(first, last, std::true_type{}) : first;
+                            for (; i <= last; ++i) visit(i, 1, bounded_tag, pow2_tag);
+                        } else {
+                            const int split = min(ifirst, last + 1);
+                            for (int i = first; i < split; ++i) visit(i, 1, bounded_tag, pow2_tag);
+                            int i = pairs ? march_pairs(ifirst, ilast, std::false_type{}) : ifirst;
+                            for (; i <= ilast; ++i) visit(i, 1, bounded_tag, pow2_tag);
+                            for (i = max(ilast + 1, split); i <= last; ++i) visit(i, 1, bounded_tag, pow2_tag);
                         }
-                        for (; i <= ilast; ++i) visit(i, 2, bounded_tag, pow2_tag);
-                        for (int i = max(ilast + 1, split); i <= last; ++i) visit(i, 1, bounded_tag, pow2_tag);
                         trailing_zero = last < S - 1;
                     }
                     };
@@ -889,70 +902,97 @@ __global__ void __launch_bounds__(kVjpBlock, vjp_min_blocks<kArith, kVol, kPose,
                         // every rounded increment is at most |vf| (1 + 2^-50) in magnitude, so the
                         // sum of a run of up to 2^31 of them stays finite in FP32
                         const bool bounded = fabs(vf) <= 1e28;
-                        int ifirst = last + 1, ilast = last;
-                        if (!kVol || bounded)
-                            interior_run(first, last, [&](int i) {
-                                double position, p[3];
-                                point_at(i, position, p);
-                                return p[0] >= 0.0 && p[0] < mx && p[1] >= 0.0 && p[1] < my && p[2] >= 0.0 && p[2] < mz;
-                            }, ifirst, ilast);
-                        const int split = min(ifirst, last + 1);
-                        for (int i = first; i < split; ++i) visit(i, true);
-                        // The interior run: no clamp, slope masks 1, no test of an increment, no
-                        // conversion of a coordinate; corners reload and run sums restart without
-                        // a branch as in the FP32 pairs.  16 views of the 256^3 / 512^2 / S = 1024
-                        // scan: pose 27.3 -> 23.0 ms (FP64 pipe 69 %), scatter 17.9 -> 15.2 (its
-                        // eight roundings to FP32 per sample take the conversion pipe).
-                        if (kVol && pending < 0 && ifirst <= ilast) {
+                        int ifirst, ilast;
+                        const bool separate = short_margins(first, last, [&](int i) {
                             double position, p[3];
-                            point_at(ifirst, position, p);
-                            pending = (interior_axis64(p[2]).lower * dims.ny + interior_axis64(p[1]).lower) * dims.nx +
-                                      interior_axis64(p[0]).lower;
-                        }
-                        double sample = (double)ifirst + 0.5;
+                            point_at(i, position, p);
+                            return p[0] >= 0.0 && p[0] < mx && p[1] >= 0.0 && p[1] < my && p[2] >= 0.0 && p[2] < mz;
+                        }, ifirst, ilast);
                         float corners[8];
                         int held = -1;
 #pragma unroll
                         for (int c = 0; c < 8; ++c) corners[c] = 0.0f;
-                        for (int i = ifirst; i <= ilast; ++i) {
-                            const double position = fma(sample, step, iv.lower);
-                            const Axis64 X = interior_axis64(fma(position, r.direction[0], r.origin[0]));
-                            const Axis64 Y = interior_axis64(fma(position, r.direction[1], r.origin[1]));
-                            const Axis64 Z = interior_axis64(fma(position, r.direction[2], r.origin[2]));
-                            const int cell = (Z.lower * dims.ny + Y.lower) * dims.nx + X.lower;
-                            const double fx = X.fraction, fy = Y.fraction, fz = Z.fraction;
-                            if (kPose) {
-                                const double alpha = power_of_two ? sample * inverse_samples : sample / (double)S;
-                                f.refresh(cell, held, X.lower, Y.lower, Z.lower, corners);
-                                held = cell;
-                                double v[8], gs[3];
-#pragma unroll
-                                for (int c = 0; c < 8; ++c) v[c] = (double)corners[c];
-                                mean = mean + interpolate64(fx, fy, fz, v);
-                                interior_slope64(fx, fy, fz, v, gs);
-#pragma unroll
-                                for (int k = 0; k < 3; ++k) {
-                                    dO[k] = dO[k] + gs[k];
-                                    dD[k] = fma(position, gs[k], dD[k]);
+                        // Samples of the inside run (kClamped) or of its interior (no clamp, slope
+                        // masks 1): no test of an increment, no conversion of a coordinate;
+                        // corners reload and run sums restart without a branch as in the FP32
+                        // pairs.  16 views of the 256^3 / 512^2 / S = 1024 scan: pose moments 27.3
+                        // -> 19.4 ms (bound by the FP64 pipe), scatter 17.9 -> 11.3 (its eight
+                        // roundings to FP32 per sample take the conversion pipe).
+                        auto march = [&](int i, int end, auto clamped_tag) {
+                            constexpr bool kClamped = decltype(clamped_tag)::value;
+                            auto axes = [&](const double* p, Axis64& X, Axis64& Y, Axis64& Z) {
+                                if constexpr (kClamped) {
+                                    X = clamped_axis64(p[0], mx, dims.cx);
+                                    Y = clamped_axis64(p[1], my, dims.cy);
+                                    Z = clamped_axis64(p[2], mz, dims.cz);
+                                } else {
+                                    X = interior_axis64(p[0]);
+                                    Y = interior_axis64(p[1]);
+                                    Z = interior_axis64(p[2]);
                                 }
-                                const double along =
-                                    fma(gs[2], r.direction[2], fma(gs[1], r.direction[1], gs[0] * r.direction[0]));
-                                sl = fma(1.0 - alpha, along, sl);
-                                su = fma(alpha, along, su);
+                                return (Z.lower * dims.ny + Y.lower) * dims.nx + X.lower;
+                            };
+                            Axis64 X, Y, Z;
+                            if (kVol && pending < 0 && i <= end) {
+                                double position, p[3];
+                                point_at(i, position, p);
+                                pending = axes(p, X, Y, Z);
                             }
-                            if (kVol) {
-                                red_add_run(acc, pending, cell, cs);
-                                const float keep = cell == pending ? 1.0f : 0.0f;
-                                pending = cell;
-                                const double px = vf * fx, qx = vf * (1.0 - fx), ay = 1.0 - fy, az = 1.0 - fz;
-                                const double plane[4] = {qx * ay, px * ay, qx * fy, px * fy};
+                            double sample = (double)i + 0.5;
+                            for (; i <= end; ++i) {
+                                const double position = fma(sample, step, iv.lower);
+                                double p[3];
 #pragma unroll
-                                for (int c = 0; c < 8; ++c)
-                                    cs[c] = fmaf(cs[c], keep, (float)(plane[c & 3] * ((c & 4) ? fz : az)));
+                                for (int k = 0; k < 3; ++k) p[k] = fma(position, r.direction[k], r.origin[k]);
+                                const int cell = axes(p, X, Y, Z);
+                                const double fx = X.fraction, fy = Y.fraction, fz = Z.fraction;
+                                if (kPose) {
+                                    const double alpha = power_of_two ? sample * inverse_samples : sample / (double)S;
+                                    f.refresh(cell, held, X.lower, Y.lower, Z.lower, corners);
+                                    held = cell;
+                                    double v[8], gs[3];
+#pragma unroll
+                                    for (int c = 0; c < 8; ++c) v[c] = (double)corners[c];
+                                    mean = mean + interpolate64(fx, fy, fz, v);
+                                    if constexpr (kClamped)
+                                        slope64(fx, fy, fz, v, p[0] >= 0.0 && p[0] < mx ? 1.0 : 0.0,
+                                                p[1] >= 0.0 && p[1] < my ? 1.0 : 0.0,
+                                                p[2] >= 0.0 && p[2] < mz ? 1.0 : 0.0, gs);
+                                    else
+                                        interior_slope64(fx, fy, fz, v, gs);
+#pragma unroll
+                                    for (int k = 0; k < 3; ++k) {
+                                        dO[k] = dO[k] + gs[k];
+                                        dD[k] = fma(position, gs[k], dD[k]);
+                                    }
+                                    const double along =
+                                        fma(gs[2], r.direction[2], fma(gs[1], r.direction[1], gs[0] * r.direction[0]));
+                                    sl = fma(1.0 - alpha, along, sl);
+                                    su = fma(alpha, along, su);
+                                }
+                                if (kVol) {
+                                    red_add_run(acc, pending, cell, cs);
+                                    const float keep = cell == pending ? 1.0f : 0.0f;
+                                    pending = cell;
+                                    const double px = vf * fx, qx = vf * (1.0 - fx), ay = 1.0 - fy, az = 1.0 - fz;
+                                    const double plane[4] = {qx * ay, px * ay, qx * fy, px * fy};
+#pragma unroll
+                                    for (int c = 0; c < 8; ++c)
+                                        cs[c] = fmaf(cs[c], keep, (float)(plane[c & 3] * ((c & 4) ? fz : az)));
+                                }
+                                sample = sample + 1.0;
                             }
-                            sample = sample + 1.0;
+                        };
+                        if (kVol && !bounded) {
+                            for (int i = first; i <= last; ++i) visit(i, true);
+                        } else if (any_in_warp(!separate)) {
+                            march(first, last, std::true_type{});
+                        } else {
+                            const int split = min(ifirst, last + 1);
+                            march(first, split - 1, std::true_type{});
+                            march(ifirst, ilast, std::false_type{});
+                            march(max(ilast + 1, split), last, std::true_type{});
                         }
-                        for (int i = max(ilast + 1, split); i <= last; ++i) visit(i, true);
                         trailing_zero = last < S - 1;
                     }
                     if (kVol && pending >= 0) flush64();

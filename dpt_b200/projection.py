@@ -468,7 +468,7 @@ class ProjectionWorkspace:
         arithmetic 101.1 ms split against 114.5 ms joint; the compensated form 65.4 ms split
         against 64.2 ms joint (its moment-storing forward costs more than the pose terms add
         to a pass bound by its scatter).  Strict FP64, 16 views:
-        forward and VJP 39 ms split, 51 ms joint."""
+        forward and VJP 31 ms split, 47 ms joint."""
         return self.spec.arith in (N.ARITH_F32, N.ARITH_F64) and self.moments_supported()
 
     def _allocate_moments(self) -> bool:
