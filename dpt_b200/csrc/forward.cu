@@ -28,6 +28,12 @@
 #ifndef DPT_FORWARD_MIN_BLOCKS_F32
 #define DPT_FORWARD_MIN_BLOCKS_F32 6
 #endif
+// Compensated, BF16 storage, which waits on its coefficient loads: 32 views of that scan 8.2 ms at
+// nine blocks (56 registers), 8.4 at eight, 8.7 at seven, 9.1 at ten; 16 views of a 512^3 volume at
+// 0.5 mm 10.5, 11.2, 12.1 and 12.7.
+#ifndef DPT_FORWARD_MIN_BLOCKS_F32C
+#define DPT_FORWARD_MIN_BLOCKS_F32C 9
+#endif
 // Strict FP64: 16 views of that scan 10.3 ms at five blocks (94 registers), 10.2 at six, 9.9 at
 // seven (72); launches of a few waves and less gain more from the registers (8 views of 64^2 of a
 // 64^3 volume 46, 60 and 56 us, 16 views of 117 x 145 at S = 336 170, 200 and 216 us).
@@ -43,6 +49,7 @@ constexpr int forward_min_blocks()
 {
     return kArith == DPT_ARITH_F32 ? DPT_FORWARD_MIN_BLOCKS_F32
          : kArith == DPT_ARITH_F64 ? DPT_FORWARD_MIN_BLOCKS_F64
+         : kArith == DPT_ARITH_F32C ? DPT_FORWARD_MIN_BLOCKS_F32C
                                    : 0;
 }
 

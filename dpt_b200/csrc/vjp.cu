@@ -25,11 +25,9 @@
 #define DPT_VJP_REUSE 0
 #endif
 // Resident blocks per SM the register allocation must allow, per arithmetic (128-thread
-// blocks).  The compensated form's cell walk measured 0.71 ms per 512^2 view (S = 1024) at four
-// blocks (118 registers), 0.59 at eight (64 registers, 376 bytes spilled to L1).  The FP32
-// joint pass, without spills at four blocks (126 registers), takes 32.8 ms per 32 views of the
-// 256^3 scan, 33.0 at five and 39.9 at six (80 registers, 592 bytes spilled); 51.2 before the
-// branches left its loops.
+// blocks).  The FP32 joint pass, without spills at four blocks (126 registers), takes 32.8 ms per
+// 32 views of the 256^3 scan, 33.0 at five and 39.9 at six (80 registers, 592 bytes spilled); 51.2
+// before the branches left its loops.
 #ifndef DPT_VJP_MIN_BLOCKS_F32
 #define DPT_VJP_MIN_BLOCKS_F32 4
 #endif
@@ -38,23 +36,26 @@
 #ifndef DPT_VJP_MIN_BLOCKS_F32_VOLUME
 #define DPT_VJP_MIN_BLOCKS_F32_VOLUME 6
 #endif
+// The compensated volume scatter, bound by its reductions: 13.5 to 13.6 ms per 32 views at five to
+// nine blocks; launches of a few waves run best at five and six (16 views of 117 x 145 at S = 336
+// 124 us, 129 at seven, 139 at eight).
 #ifndef DPT_VJP_MIN_BLOCKS_F32C
-#define DPT_VJP_MIN_BLOCKS_F32C 8
+#define DPT_VJP_MIN_BLOCKS_F32C 6
 #endif
 // FP32 pose moments: alpha_i = (i + 0.5) / S as one multiplication by 1/S when S is a power
 // of two (both exact), else from a per-block table of IEEE quotients
 #ifndef DPT_VJP_POW2_ALPHA
 #define DPT_VJP_POW2_ALPHA 1
 #endif
-// The compensated form's forward that stores the pose moments (no scatter) measured 158.6 ->
-// 153.4 ms per 360-view full scan at nine blocks (56 registers), 155.4 at ten.
+// The compensated form's forward that stores the pose moments (no scatter): 10.9 ms per 32 views
+// of the full scan at eight blocks (64 registers), 11.1 at seven, 11.6 at nine.
 #ifndef DPT_VJP_MIN_BLOCKS_F32C_FORWARD
-#define DPT_VJP_MIN_BLOCKS_F32C_FORWARD 9
+#define DPT_VJP_MIN_BLOCKS_F32C_FORWARD 8
 #endif
-// The compensated joint volume + pose pass: 237.9 ms per full scan at eight blocks (64
-// registers, 376 bytes spilled), 247.3 at seven, 252.6 at six, 249.7 at nine, 310.3 at ten.
+// The compensated joint volume + pose pass, per 32 views: 17.2 ms at seven blocks (72 registers,
+// 348 bytes spilled), 17.6 at six, 18.1 at eight, 18.4 at five.
 #ifndef DPT_VJP_MIN_BLOCKS_F32C_JOINT
-#define DPT_VJP_MIN_BLOCKS_F32C_JOINT 8
+#define DPT_VJP_MIN_BLOCKS_F32C_JOINT 7
 #endif
 // The FP32 forward that stores the pose moments (per 32 views of the full scan): 23.9 ms at
 // four blocks, 23.6 at five, and with more spilled 25.0 at six (80 registers), 25.8 at seven.
@@ -1094,7 +1095,7 @@ __global__ void __launch_bounds__(kVjpBlock, vjp_min_blocks<kArith, kVol, kPose,
                         if (first <= last) {
                             walk_cells(dims, entry, sv, first, last, [&](const CellRun& run) {
                                 const float dx = run.d[0], dy = run.d[1], dz = run.d[2];
-                                const float dxy = dx * dy, dxz = dx * dz, dyz = dy * dz;
+                                const float dxy = run.dxy, dxz = run.dxz, dyz = run.dyz;
                                 const float nf = run.nf, s1 = run.s1, s2 = run.s2, s3 = run.s3;
                                 if (kPose) {
                                     PolyCache<Field, false> cell;
@@ -1105,7 +1106,7 @@ __global__ void __launch_bounds__(kVjpBlock, vjp_min_blocks<kArith, kVol, kPose,
                                     float g1[3] = {fmaf(o.t1, dz, o.a * dy), fmaf(o.t2, dz, o.a * dx),
                                                    fmaf(o.t2, dy, o.t1 * dx)};
                                     float g2[3] = {o.c7 * dyz, o.c7 * dxz, o.c7 * dxy};
-                                    const float offset = (float)run.i0 + 0.5f;
+                                    const float offset = run.offset;
 #pragma unroll
                                     for (int k = 0; k < 3; ++k) {
                                         if (!((run.interior >> k) & 1)) g0[k] = g1[k] = g2[k] = 0.0f;
@@ -1126,7 +1127,7 @@ __global__ void __launch_bounds__(kVjpBlock, vjp_min_blocks<kArith, kVol, kPose,
                                     m[4] = fmaf(s2, dxy, fmaf(s1, fmaf(fx, dy, fy * dx), nf * fxy));
                                     m[5] = fmaf(s2, dxz, fmaf(s1, fmaf(fx, dz, fz * dx), nf * fxz));
                                     m[6] = fmaf(s2, dyz, fmaf(s1, fmaf(fy, dz, fz * dy), nf * fyz));
-                                    m[7] = fmaf(s3, dxy * dz,
+                                    m[7] = fmaf(s3, run.dxyz,
                                                 fmaf(s2, fmaf(fz, dxy, fmaf(fy, dxz, fx * dyz)),
                                                      fmaf(s1, fmaf(fyz, dx, fmaf(fxz, dy, fxy * dz)),
                                                           nf * (fxy * fz))));
