@@ -21,6 +21,7 @@
 // Poisson trial domain.
 #include <cstdint>
 #include <initializer_list>
+#include <type_traits>
 
 #include "launch.h"
 
@@ -460,8 +461,15 @@ __global__ void __launch_bounds__(kTile) k_objective(const TIn* __restrict__ pre
                     derivative = 1.0;
                 } else {
                     if (isfinite(predicted) && predicted <= 0.0) bits |= 8;
-                    derivative = difference / predicted;
-                    loss = poisson_half_deviance(predicted, observed);
+                    // A loss without a seed needs no derivative.  A seed without a loss needs no
+                    // deviance where that is known to be finite (positive FP32 operands below
+                    // 2^128: the weighted terms stay far inside the FP64 range), except to flag a
+                    // weight that is not, which the seed then does itself.  The kernel is bound by
+                    // FP64 arithmetic, 3 divisions and a logarithm or series per pixel.
+                    if (seed) derivative = difference / predicted;
+                    const bool finite_loss = std::is_same_v<TIn, float> && predicted > 0.0 && observed > 0.0 &&
+                                             isfinite(predicted) && isfinite(observed);
+                    loss = partials || !finite_loss ? poisson_half_deviance(predicted, observed) : 0.0;
                 }
             }
             if (kWide && !poisson)
