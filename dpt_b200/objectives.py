@@ -90,6 +90,10 @@ class ObjectiveWorkspace:
         """Deliver and reset one completed checkpoint, including reported errors."""
         self._raise(self.status.read(self._stream(), reset=True))
 
+    def settle(self) -> None:
+        """``consume_status`` where a launch may have reported since the last clean checkpoint."""
+        self._raise(self.status.pending(self._stream(), reset=True))
+
     def _raise(self, code: int) -> None:
         rule = "unmasked observations must be finite"
         if self.spec.kind == "poisson":
@@ -115,7 +119,7 @@ class ObjectiveWorkspace:
             raise ContractError("valid requires a masked objective specification")
 
     def _check(self, stream, prediction, observation, weights, valid, size: int) -> None:
-        self._raise(self.status.read(stream))
+        self._raise(self.status.pending(stream))
         if size:
             dtype = N.F64 if prediction is not None and prediction.dtype == torch.float64 else N.F32
             D.call(N.library().dpt_b200_objective_check(

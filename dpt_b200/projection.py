@@ -166,7 +166,14 @@ def _ptr(tensor: torch.Tensor | None) -> int | None:
 
 
 def _stream(device: torch.device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    """Handle of the device's current stream (without the stream object around it)."""
+    index = torch.cuda.current_device() if device.index is None else device.index
+    return torch._C._cuda_getCurrentRawStream(index)
+
+
+def _on(device: torch.device):
+    """``torch.cuda.device(device)``, or nothing where that device is already the current one."""
+    return contextlib.nullcontext() if torch.cuda.current_device() == device.index else torch.cuda.device(device)
 
 
 class FieldCopies:
@@ -506,7 +513,7 @@ class ProjectionWorkspace:
         ``moments=True`` (FP32, compensated or strict FP64 arithmetic) also stores each ray's pose moments, so that a
         following ``vjp`` with the same field and poses forms the pose gradient without
         sampling again; the image is identical either way."""
-        with self.lock, torch.cuda.device(self.device):
+        with self.lock, _on(self.device):
             field = self.check_field(field)
             poses = self.check_poses(poses)
             if out is None:
@@ -540,7 +547,7 @@ class ProjectionWorkspace:
         (``(views, 12)`` packed or ``(views, 6)`` local-right tangent)."""
         if not volume and pose is None:
             raise ContractError("request at least one projection gradient")
-        with self.lock, torch.cuda.device(self.device):
+        with self.lock, _on(self.device):
             lib = N.library()
             field = self.check_field(field)
             poses = self.check_poses(poses)
@@ -611,7 +618,7 @@ class ProjectionWorkspace:
     def pose_sensitivities(self, field: torch.Tensor, poses: torch.Tensor, cotangent: torch.Tensor,
                            *, checked: bool = True) -> torch.Tensor:
         """Per-ray rows ``cotangent[p] * dL[p]/d xi`` in local-right order, shape (rays, 6)."""
-        with self.lock, torch.cuda.device(self.device):
+        with self.lock, _on(self.device):
             field = self.check_field(field)
             poses = self.check_poses(poses)
             cot = self._cotangent(cotangent)
@@ -626,7 +633,7 @@ class ProjectionWorkspace:
 
     def counts(self, poses: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
         """Per-ray clip interval (lower, upper) and realised midpoint count."""
-        with self.lock, torch.cuda.device(self.device):
+        with self.lock, _on(self.device):
             poses = self.check_poses(poses)
             n = self.plan.rays
             lower = torch.empty(n, dtype=torch.float64, device=self.device)

@@ -113,6 +113,7 @@ class _FixedAnchor:
     def __init__(self, transform: RigidTransform) -> None:
         self.transform = transform
         self._by_device: dict[torch.device, torch.Tensor] = {}
+        self._rows: dict[torch.device, torch.Tensor] = {}
 
     def on(self, device: torch.device) -> torch.Tensor:
         packed = self._by_device.get(device)
@@ -120,6 +121,14 @@ class _FixedAnchor:
             packed = torch.tensor(self.transform.packed(), dtype=torch.float64, device=device)
             self._by_device[device] = packed
         return packed
+
+    def rows(self, device: torch.device, views: int) -> torch.Tensor:
+        """The same, one row per view (the poses of a call without a pose, copied once)."""
+        rows = self._rows.get(device)
+        if rows is None:
+            rows = self.on(device).expand(views, 12).contiguous()
+            self._rows[device] = rows
+        return rows
 
 
 class Projector(torch.nn.Module):
@@ -195,7 +204,7 @@ class Projector(torch.nn.Module):
                 raise ContractError("move the Projector anchor to the field device with .to(device)")
             ANCHOR.check(anchor, self.views)
             if pose is None:
-                packed = anchor
+                packed = anchor if self.anchor is not None else self._fixed_anchor.rows(field.device, self.views)
             else:
                 TANGENT.check(pose, self.views)
                 if pose.device != field.device:

@@ -148,7 +148,7 @@ class _TransmissionCall:
             scope.keep(result)
             _transmit(_vector(depth), self.native_beam(beam), **{_KEYWORDS[self.output][0]: _vector(result)},
                       workspace=self.workspace, stream=self.workspace.stream, validate=self.validate)
-            self.workspace.consume_status()
+            self.workspace.settle()
         return result
 
     def backward(self, depth: torch.Tensor, beam, seed: torch.Tensor, wants: tuple[bool, bool]):
@@ -161,7 +161,7 @@ class _TransmissionCall:
             transmission_vjp(_vector(depth), self.native_beam(beam), **{_KEYWORDS[self.output][1]: _vector(seed)},
                              out_grad_L=_vector(grad_depth), out_grad_n0=_vector(grad_beam),
                              workspace=self.workspace, stream=self.workspace.stream, validate=self.validate)
-            self.workspace.consume_status()
+            self.workspace.settle()
         return grad_depth, grad_beam
 
 
@@ -215,12 +215,12 @@ class _ObjectiveCall:
             evaluate_objective(_vector(prediction), _vector(observation), out_loss=result.reshape(1),
                                weights=_vector(weights), valid=_vector(valid), workspace=self.workspace,
                                stream=self.workspace.stream, validate=self.validate)
-            self.workspace.consume_status()
+            self.workspace.settle()
         return result
 
     def gradient(self, prediction, observation, weights, valid, seed: torch.Tensor) -> torch.Tensor:
         with _OnWorkspaceStream(self.workspace, (prediction, observation, weights, valid, seed)) as scope:
-            self.workspace.check_status()
+            self.workspace._raise(self.workspace.status.pending(self.workspace._stream()))
             scale = float(seed.item())
             if scale - scale != 0.0:  # NaN or infinite
                 raise ContractError("objective cotangent must be finite")
@@ -234,7 +234,7 @@ class _ObjectiveCall:
                            weights=_vector(weights), valid=_vector(valid), workspace=self.workspace,
                            stream=self.workspace.stream, validate=self.validate)
             try:
-                self.workspace.consume_status()
+                self.workspace.settle()
             except NumericalError as error:
                 # a plain range failure means the FP64 seed overflowed the prediction's dtype;
                 # typed subclasses (an input outside its domain) pass through

@@ -109,6 +109,10 @@ class TransmissionWorkspace:
         """Deliver and reset one completed checkpoint, including reported errors."""
         self._raise(self.status.read(self._stream(), reset=True))
 
+    def settle(self) -> None:
+        """``consume_status`` where a launch may have reported since the last clean checkpoint."""
+        self._raise(self.status.pending(self._stream(), reset=True))
+
     def warm(self, **_ignored) -> tuple[str, ...]:
         """Kernels are compiled ahead of time: nothing to prepare."""
         return ()
@@ -156,7 +160,7 @@ def _beam(n0, count: int, workspace: TransmissionWorkspace) -> tuple[torch.Tenso
 def _check_values(workspace: TransmissionWorkspace, stream: torch.cuda.Stream,
                   arrays: list[tuple[str, torch.Tensor | None, str]]) -> None:
     """Run the input rules on the device; on failure name the first offending element."""
-    workspace._raise(workspace.status.read(stream))
+    workspace._raise(workspace.status.pending(stream))
     lib = N.library()
     for name, array, rule in arrays:
         if array is not None and array.numel():
