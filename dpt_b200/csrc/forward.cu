@@ -44,13 +44,16 @@
 namespace dpt {
 namespace {
 
-template <int kArith>
+// Direct gathers take registers for eight addresses: the compensated form without a cap (8.4 ms per
+// 16 views, 9.6 at nine blocks), FP32 at eight (13.1 ms, 13.4 without).
+template <int kArith, class Field>
 constexpr int forward_min_blocks()
 {
-    return kArith == DPT_ARITH_F32 ? DPT_FORWARD_MIN_BLOCKS_F32
-         : kArith == DPT_ARITH_F64 ? DPT_FORWARD_MIN_BLOCKS_F64
-         : kArith == DPT_ARITH_F32C ? DPT_FORWARD_MIN_BLOCKS_F32C
-                                   : 0;
+    constexpr bool direct = std::is_same_v<Field, PlainF32>;
+    return kArith == DPT_ARITH_F32    ? (direct ? 8 : DPT_FORWARD_MIN_BLOCKS_F32)
+         : kArith == DPT_ARITH_F64    ? DPT_FORWARD_MIN_BLOCKS_F64
+         : kArith == DPT_ARITH_F32C   ? (direct ? 0 : DPT_FORWARD_MIN_BLOCKS_F32C)
+                                      : 0;
 }
 
 // FP32 sample of the field at grid point (x, y, z): zero outside the half-cell support.
@@ -520,7 +523,7 @@ __device__ __forceinline__ void forward_tile(const RayArgs& a, const Field& f, O
 }
 
 template <int kArith, class Field, typename Out>
-__global__ void __launch_bounds__(kForwardBlock, forward_min_blocks<kArith>())
+__global__ void __launch_bounds__(kForwardBlock, forward_min_blocks<kArith, Field>())
     k_forward(RayArgs a, Field f, Out* __restrict__ image)
 {
     __shared__ ViewShared vs;
@@ -550,18 +553,17 @@ struct PackedForward {
 // the whole descriptor set is one kernel parameter: 32,764 bytes at most (CUDA 12.1, Volta on)
 static_assert(sizeof(PackedForward<QuadF32>) <= 32764, "packed descriptors exceed the parameter space");
 
-// Blocks per SM the packed kernel is compiled for: the occupancy the single-problem kernel of
-// the same arithmetic reaches (its register count at 128 threads).  Indexing the descriptors
-// with a run-time problem number costs registers the single-problem kernel takes from the
-// constant bank; without the bound the FP32 form drops from 9 to 7 resident blocks and runs
-// 8 requests of 8 views of 512^2 at S = 512 in 20.1 ms against 18.6 ms with it.
+// Blocks per SM the packed kernel is compiled for: near the occupancy of the single-problem kernel
+// of the same arithmetic.  Indexing the descriptors with a run-time problem number costs registers
+// the single-problem kernel takes from the constant bank; FP32, 8 requests of 8 views of 512^2 at
+// S = 512: 17.4 ms at eight blocks, 17.7 at seven, 18.8 at six, 18.4 at nine (18.5 before the
+// sample pairs); 32 requests of 2 views of 128^2 0.64 ms (0.95).
 template <int kArith>
 constexpr int packed_min_blocks()
 {
-    return kArith == DPT_ARITH_F32 || kArith == DPT_ARITH_FAST ? 9
-         : kArith == DPT_ARITH_F64 ? 7
-         : kArith == DPT_ARITH_CELLS ? 5
-         : 8;  // compensated, mixed
+    return kArith == DPT_ARITH_FAST || kArith == DPT_ARITH_F32C ? 9
+         : kArith == DPT_ARITH_F64 || kArith == DPT_ARITH_CELLS ? 5
+                                                               : 8;  // FP32, mixed
 }
 
 template <int kArith, class Field, typename Out>
