@@ -511,8 +511,8 @@ def run_gpu(args) -> None:
         "peak_source": "measured in this run: dpt_b200_read_probe, float4 .cg loads of a 64 MiB L2-resident "
                        "buffer, best of 10 launches of 20 passes",
         "bytes_per_sample": algorithmic_bytes(dominant, storage_bytes),
-        "limiter": "FP32 pipe (ncu on the forward with pose moments: FMA pipe 65.6% of active cycles, "
-                   "math-pipe throttle the top stall; L1 hit 92.7%, L2 hit 86.8%, DRAM 0.21 B per realised sample)",
+        "limiter": "FP32 pipe (ncu on the forward with pose moments: FMA pipe 66.5% of active cycles, "
+                   "math-pipe throttle the top stall; L1 hit 79.2%, L2 hit 85.8%, DRAM 0.21 B per realised sample)",
         "hbm": {"peak": hbm_peak, "peak_source": f"{hbm_kind} MEASURED_PEAKS hbm_gbs",
                 "dram_gbs": None if traffic is None else round(traffic / (mean_ms * 1e-3) / 1e9, 1),
                 "frac": None if traffic is None else round(traffic / (mean_ms * 1e-3) / 1e9 / hbm_peak, 4)},
