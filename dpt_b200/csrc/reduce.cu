@@ -22,26 +22,25 @@ __global__ void __launch_bounds__(256) k_finish_pose(int view_begin, int tiles, 
                                                      double* __restrict__ gradient,
                                                      int accumulate, int32_t* status)
 {
+    // a block per (view, component): with one block walking a view's components in turn the
+    // reduction of two views took 20 us
     __shared__ double tree[256];
-    const int view = blockIdx.x;
+    const int view = blockIdx.x, k = blockIdx.y;
     const double* base = partials + (int64_t)view * tiles * components;
-    for (int k = 0; k < components; ++k) {
-        double s = 0.0;
-        for (int b = threadIdx.x; b < tiles; b += 256) s += base[(int64_t)b * components + k];
-        tree[threadIdx.x] = s;
+    double s = 0.0;
+    for (int b = threadIdx.x; b < tiles; b += 256) s += base[(int64_t)b * components + k];
+    tree[threadIdx.x] = s;
+    __syncthreads();
+    for (int width = 128; width > 0; width >>= 1) {
+        if (threadIdx.x < width) tree[threadIdx.x] += tree[threadIdx.x + width];
         __syncthreads();
-        for (int width = 128; width > 0; width >>= 1) {
-            if (threadIdx.x < width) tree[threadIdx.x] += tree[threadIdx.x + width];
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) {
-            double value = tree[0];
-            double* out = gradient + (int64_t)view * components + k;
-            if (accumulate) value += *out;
-            *out = value;
-            if (!isfinite(value)) atomicOr(status + view_begin + view, 2);
-        }
-        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        double value = tree[0];
+        double* out = gradient + (int64_t)view * components + k;
+        if (accumulate) value += *out;
+        *out = value;
+        if (!isfinite(value)) atomicOr(status + view_begin + view, 2);
     }
 }
 
@@ -140,7 +139,7 @@ cudaError_t launch_finish_pose(int view_begin, int view_count, int tiles, int co
                                const double* partials, double* gradient, int accumulate,
                                int32_t* status, cudaStream_t stream)
 {
-    k_finish_pose<<<view_count, 256, 0, stream>>>(view_begin, tiles, components, partials,
+    k_finish_pose<<<dim3((unsigned)view_count, (unsigned)components), 256, 0, stream>>>(view_begin, tiles, components, partials,
                                                   gradient, accumulate, status);
     return cudaGetLastError();
 }
