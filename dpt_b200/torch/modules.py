@@ -108,27 +108,25 @@ TANGENT = _PoseRule("pose", 6)
 
 
 class _FixedAnchor:
-    """A host ``RigidTransform`` anchor, materialised as a packed FP64 tensor once per device."""
+    """A host ``RigidTransform`` anchor, materialised as a packed FP64 tensor once per device and
+    row count (0: the unbatched pose).
+
+    Any later call may read the tensor, on any stream and under autograd, so it is built on the host
+    and uploaded by a copy that has ended when it returns (a kernel that wrote it would be ordered
+    after nothing but its own stream), outside inference mode."""
 
     def __init__(self, transform: RigidTransform) -> None:
         self.transform = transform
-        self._by_device: dict[torch.device, torch.Tensor] = {}
-        self._rows: dict[torch.device, torch.Tensor] = {}
+        self._uploaded: dict[tuple[torch.device, int], torch.Tensor] = {}
 
-    def on(self, device: torch.device) -> torch.Tensor:
-        packed = self._by_device.get(device)
+    def on(self, device: torch.device, rows: int = 0) -> torch.Tensor:
+        packed = self._uploaded.get((device, rows))
         if packed is None:
-            packed = torch.tensor(self.transform.packed(), dtype=torch.float64, device=device)
-            self._by_device[device] = packed
+            values = self.transform.packed()
+            with torch.inference_mode(False):
+                packed = torch.tensor([values] * rows if rows else values, dtype=torch.float64, device=device)
+            self._uploaded[device, rows] = packed
         return packed
-
-    def rows(self, device: torch.device, views: int) -> torch.Tensor:
-        """The same, one row per view (the poses of a call without a pose, copied once)."""
-        rows = self._rows.get(device)
-        if rows is None:
-            rows = self.on(device).expand(views, 12).contiguous()
-            self._rows[device] = rows
-        return rows
 
 
 class Projector(torch.nn.Module):
@@ -204,7 +202,7 @@ class Projector(torch.nn.Module):
                 raise ContractError("move the Projector anchor to the field device with .to(device)")
             ANCHOR.check(anchor, self.views)
             if pose is None:
-                packed = anchor if self.anchor is not None else self._fixed_anchor.rows(field.device, self.views)
+                packed = anchor if self.anchor is not None else self._fixed_anchor.on(field.device, self.views)
             else:
                 TANGENT.check(pose, self.views)
                 if pose.device != field.device:

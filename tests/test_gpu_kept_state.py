@@ -1,0 +1,51 @@
+"""State kept between calls on the GPU: poses used from several streams, status words read across
+streams and graph replays, and pose moments beside a caller's own memory."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+from dpt_b200.torch import Projector
+from scenes import cone_scene
+
+pytestmark = pytest.mark.gpu
+DEVICE = "cuda:0"
+
+
+def busy(stream: torch.cuda.Stream) -> None:
+    """Queue some tens of milliseconds of products on a stream."""
+    with torch.cuda.stream(stream):
+        a = torch.ones((4096, 4096), device=DEVICE)
+        for _ in range(20):
+            a = a @ a * 1e-4
+
+
+def test_one_projector_on_two_streams_without_a_pose():
+    grid, geometry, values = cone_scene(views=3)
+    field = torch.tensor(values, dtype=torch.float32, device=DEVICE)
+    expected = Projector(grid=grid, geometry=geometry, samples_per_ray=64)(field)
+    shared = Projector(grid=grid, geometry=geometry, samples_per_ray=64)
+    first, second = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    busy(first)
+    with torch.cuda.stream(first):
+        poses = shared._packed_poses(field, None, None)  # made behind the queued work
+    with torch.cuda.stream(second):
+        torch.testing.assert_close(shared(field), expected, rtol=0, atol=0)
+    with torch.cuda.stream(first):
+        torch.testing.assert_close(shared(field), expected, rtol=0, atol=0)
+    assert shared._packed_poses(field, None, None) is poses
+
+
+def test_projector_first_called_in_inference_mode_trains():
+    grid, geometry, values = cone_scene(views=3)
+    field = torch.tensor(values, dtype=torch.float32, device=DEVICE)
+    projector = Projector(grid=grid, geometry=geometry, samples_per_ray=64)
+    with torch.inference_mode():
+        expected = projector(field)
+    volume = field.clone().requires_grad_()
+    image = projector(volume)
+    image.sum().backward()
+    torch.testing.assert_close(image.detach(), expected.clone(), rtol=0, atol=0)
+    assert float(volume.grad.abs().sum()) > 0
