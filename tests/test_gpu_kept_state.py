@@ -6,7 +6,9 @@ from __future__ import annotations
 import pytest
 import torch
 
+from dpt_b200.contracts import NumericalError
 from dpt_b200.torch import Projector
+from dpt_b200.transmission import TransmissionSpec, prepare_transmission, transmission_vjp, transmit
 from scenes import cone_scene
 
 pytestmark = pytest.mark.gpu
@@ -49,3 +51,22 @@ def test_projector_first_called_in_inference_mode_trains():
     image.sum().backward()
     torch.testing.assert_close(image.detach(), expected.clone(), rtol=0, atol=0)
     assert float(volume.grad.abs().sum()) > 0
+
+
+def test_an_error_on_an_owned_side_stream_reaches_its_checkpoint_once():
+    side = torch.cuda.Stream()
+    ws = prepare_transmission(TransmissionSpec(beam="scalar"), device=DEVICE, max_pixels=300, stream=side)
+    depth, seed = torch.zeros(300, device=DEVICE), torch.full((300,), 1e38, device=DEVICE)
+    out, gradient = torch.empty_like(depth), torch.empty_like(depth)
+    torch.cuda.synchronize()
+    busy(side)
+    # -n0 exp(-L) seed is beyond FP32; the current stream is another one and idle
+    transmission_vjp(depth, 1e5, cotangent_counts=seed, out_grad_L=gradient, workspace=ws, validate=False)
+    with pytest.raises(NumericalError):
+        ws.check_status()
+    transmit(depth, 1e5, out_T=out, workspace=ws, validate=False)
+    with pytest.raises(NumericalError):
+        ws.settle()
+    ws.settle()
+    ws.check_status()
+    torch.testing.assert_close(out, torch.ones_like(out), rtol=0, atol=0)

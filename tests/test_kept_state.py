@@ -3,10 +3,13 @@ is complete when it is stored, and is ordered after the stream that wrote it."""
 
 from __future__ import annotations
 
+import contextlib
+
 import pytest
 import torch
 from torch.utils._python_dispatch import TorchDispatchMode
 
+from dpt_b200._device import StatusWord
 from dpt_b200.geometry import RigidTransform
 from dpt_b200.torch import Projector
 from scenes import cone_scene
@@ -53,3 +56,72 @@ def test_poses_first_used_in_inference_mode_can_be_saved_for_backward():
         projector._packed_poses(field, torch.zeros(6, dtype=torch.float64), None)
     assert not projector._packed_poses(field, None, None).is_inference()
     assert not projector._anchor_on(field.device).is_inference()
+
+
+class FakeStream:
+    def __init__(self, handle: int) -> None:
+        self.cuda_stream = handle
+
+    def synchronize(self) -> None:
+        pass
+
+
+@pytest.fixture
+def word(monkeypatch):
+    """A status word on the host with stand-in streams; ``copies`` lists the stream each readback
+    was queued on."""
+    at = [1]
+
+    @contextlib.contextmanager
+    def stream(s):
+        at.append(s.cuda_stream)
+        yield
+        at.pop()
+
+    zeros = torch.zeros
+    monkeypatch.setattr(torch, "zeros", lambda *a, pin_memory=False, **k: zeros(*a, **k))
+    monkeypatch.setattr(torch.cuda, "stream", stream)
+    monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", lambda device: at[-1], raising=False)
+    status = StatusWord(torch.device("cpu"))
+    status.copies = []
+    copy = status.host.copy_
+
+    class Host:
+        def copy_(self, source, non_blocking=False):
+            status.copies.append(at[-1])
+            return copy(source)
+
+        def __getitem__(self, index):
+            return status.host_values[index]
+
+    status.host_values, status.host = status.host, Host()
+    return status
+
+
+def test_status_word_is_read_on_the_stream_that_writes_it(word):
+    side = FakeStream(2)
+    with word.launch(side) as address:
+        assert address == word.word.data_ptr()
+    word.word.fill_(8)
+    assert word.read(side) == 8 and word.pending(side) == 8  # sticky until reset
+    assert word.pending(side, reset=True) == 8 and word.pending(side) == 0
+    assert int(word.word) == 0 and word.copies == [2, 2, 2]
+
+
+def test_status_word_stays_pending_until_its_own_stream_was_read_clean(word):
+    side, other = FakeStream(2), FakeStream(3)
+    assert word.pending(side) == 0 and word.copies == []  # no launch: no wait
+    with word.launch(side):
+        word.read(side)  # another thread's read before the launch is queued
+    assert word.pending(side) == 0 and word.copies == [2, 2]
+    with word.launch(side):
+        pass
+    word.read(other)  # ordered after another stream only
+    word.clear(other)
+    word.word.fill_(2)  # the launch reports now
+    assert word.pending(other) == 2
+    word.ptr  # given away: launches that are not followed
+    word.read(side, reset=True)
+    word.read(other)
+    word.copies.clear()
+    assert word.pending(side) == 0 and word.copies == [2]
