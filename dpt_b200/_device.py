@@ -46,7 +46,7 @@ class StatusWord:
         self.host = torch.zeros(1, dtype=torch.int32, pin_memory=True)
         self._lock = threading.Lock()
         self._unread: dict[int, int] = {}  # stream handle -> count of launches since a clean read
-        self._untracked = False  # whether the word's address was given away
+        self._untracked = False  # whether the word's address was given away, or captured
 
     @property
     def ptr(self) -> int:
@@ -55,13 +55,20 @@ class StatusWord:
         self._untracked = True
         return self.word.data_ptr()
 
+    def _capturing(self, stream: torch.cuda.Stream) -> bool:
+        with current(stream, self.device):
+            return torch.cuda.is_current_stream_capturing()
+
     def _count(self, stream: torch.cuda.Stream) -> None:
         with self._lock:
             self._unread[stream.cuda_stream] = self._unread.get(stream.cuda_stream, 0) + 1
 
     @contextlib.contextmanager
     def launch(self, stream: torch.cuda.Stream):
-        """The word's address for one call that queues its work on `stream` in this block."""
+        """The word's address for one call that queues its work on `stream` in this block.  Under
+        capture every replay of the graph may report, unseen from here."""
+        if self._capturing(stream):
+            self._untracked = True
         self._count(stream)
         try:
             yield self.word.data_ptr()
@@ -70,8 +77,10 @@ class StatusWord:
 
     def pending(self, stream: torch.cuda.Stream, *, reset: bool = False) -> int:
         """``read`` where a launch may have reported since the last clean read, else 0 without
-        waiting for the stream."""
-        return self.read(stream, reset=reset) if self._unread or self._untracked else 0
+        waiting for the stream.  (A capture refuses a checkpoint, whether or not it has to wait.)"""
+        if self._unread or self._untracked or self._capturing(stream):
+            return self.read(stream, reset=reset)
+        return 0
 
     def read(self, stream: torch.cuda.Stream, *, reset: bool = False) -> int:
         """Synchronise `stream` and return the word; with `reset`, clear it afterwards."""

@@ -6,8 +6,10 @@ from __future__ import annotations
 import pytest
 import torch
 
-from dpt_b200.contracts import NumericalError
+from dpt_b200.contracts import NumericalError, TrialDomainError
+from dpt_b200.objectives import ObjectiveSpec, evaluate_objective, prepare_objective
 from dpt_b200.torch import Projector
+from dpt_b200.torch.operators import objective
 from dpt_b200.transmission import TransmissionSpec, prepare_transmission, transmission_vjp, transmit
 from scenes import cone_scene
 
@@ -70,3 +72,33 @@ def test_an_error_on_an_owned_side_stream_reaches_its_checkpoint_once():
     ws.settle()
     ws.check_status()
     torch.testing.assert_close(out, torch.ones_like(out), rtol=0, atol=0)
+
+
+def test_an_error_of_a_replayed_graph_reaches_the_next_operator():
+    ws = prepare_objective(ObjectiveSpec(kind="poisson", domain="counts"), device=DEVICE, max_pixels=300)
+    observation = torch.full((300,), 5.0, device=DEVICE)
+    prediction = torch.full((300,), 4.0, device=DEVICE)
+    loss = torch.empty(1, dtype=torch.float64, device=DEVICE)
+
+    def checked():
+        mu = torch.full((300,), 4.0, device=DEVICE, requires_grad=True)
+        return mu, objective(mu, observation, workspace=ws)
+
+    evaluate_objective(prediction, observation, out_loss=loss, workspace=ws, validate=False)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        evaluate_objective(prediction, observation, out_loss=loss, workspace=ws, validate=False)
+    graph.replay()
+    mu, value = checked()
+    prediction.fill_(-1.0)
+    graph.replay()
+    with pytest.raises(TrialDomainError):  # a zero cotangent launches nothing of its own
+        (0.0 * value).backward()
+    with pytest.raises(TrialDomainError):
+        checked()
+    ws.clear_status()
+    mu, value = checked()
+    value.backward()
+    assert float(mu.grad.abs().sum()) > 0
+    del graph

@@ -58,6 +58,9 @@ def test_poses_first_used_in_inference_mode_can_be_saved_for_backward():
     assert not projector._anchor_on(field.device).is_inference()
 
 
+CAPTURING = 9  # handle of the stand-in stream that captures
+
+
 class FakeStream:
     def __init__(self, handle: int) -> None:
         self.cuda_stream = handle
@@ -81,6 +84,7 @@ def word(monkeypatch):
     zeros = torch.zeros
     monkeypatch.setattr(torch, "zeros", lambda *a, pin_memory=False, **k: zeros(*a, **k))
     monkeypatch.setattr(torch.cuda, "stream", stream)
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: at[-1] == CAPTURING)
     monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", lambda device: at[-1], raising=False)
     status = StatusWord(torch.device("cpu"))
     status.copies = []
@@ -123,5 +127,17 @@ def test_status_word_stays_pending_until_its_own_stream_was_read_clean(word):
     word.ptr  # given away: launches that are not followed
     word.read(side, reset=True)
     word.read(other)
+    word.copies.clear()
+    assert word.pending(side) == 0 and word.copies == [2]
+
+
+def test_status_word_a_graph_was_given_is_read_at_every_checkpoint(word):
+    side, capturing = FakeStream(2), FakeStream(CAPTURING)
+    assert word.pending(capturing) == 0 and word.copies == [CAPTURING]  # where a real one refuses
+    with word.launch(capturing):
+        pass
+    assert word.read(capturing) == 0 and word.read(side) == 0
+    word.word.fill_(8)  # a replay reports
+    assert word.pending(side, reset=True) == 8
     word.copies.clear()
     assert word.pending(side) == 0 and word.copies == [2]
