@@ -44,7 +44,7 @@ from .geometry import compose_pose
 _CACHE_LIMIT = 8
 _CACHE: OrderedDict[tuple, ProjectionWorkspace] = OrderedDict()
 _CACHE_LOCK = RLock()
-_TAGS = (torch.Tag.cudagraph_unsafe,)
+_TAGS = (torch.Tag.cudagraph_unsafe,)  # custom_op adds pt2_compliant_tag
 _KINDS = {DetectorGeometry: "cone", ParallelGeometry: "parallel", CurvedDetectorGeometry: "curved"}
 _CONSTRUCTORS = {"cone": DetectorGeometry, "parallel": ParallelGeometry, "curved": CurvedDetectorGeometry}
 _FIELD_DTYPES = (torch.float32, torch.float16, torch.bfloat16)
@@ -187,7 +187,7 @@ def _functional(name: str, schema: str, body) -> torch._ops.OpOverload:
     """The operator ``dpt::name`` of a body that returns new tensors.  Defined through the library
     directly: the wrapper ``custom_op`` puts around a body costs 20 us a call, a fifth of a small
     forward (8 views of 64^2)."""
-    torch.library.define(f"dpt::{name}", schema, tags=_TAGS)
+    torch.library.define(f"dpt::{name}", schema, tags=(torch.Tag.pt2_compliant_tag, *_TAGS))
     torch.library.impl(f"dpt::{name}", "default", body)
     return getattr(torch.ops.dpt, name).default
 
@@ -246,6 +246,14 @@ def _vjp_fake(field, poses, cotangent, value, active_volume, active_pose):
         field.new_empty(field.shape if active_volume else (0,)),
         poses.new_empty(poses.shape if active_pose else (0,)),
     )
+
+
+def _vjp_backward(ctx, *cotangents):
+    raise RuntimeError("dpt::project_vjp has no derivative formula: projection gradients are first order")
+
+
+# without a formula of its own the operator would only warn and leave its inputs without a gradient
+torch.library.register_autograd("dpt::project_vjp", _vjp_backward)
 
 
 def _setup_context(ctx, inputs, output):

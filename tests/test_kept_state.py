@@ -1,5 +1,6 @@
-"""State kept between calls, where no GPU is needed to show it sound: what every later call may read
-is complete when it is stored, and is ordered after the stream that wrote it."""
+"""State kept between calls, and the operators' registration, where no GPU is needed to show them
+sound: what a later call may read is complete when it is stored, and is ordered after the stream that
+wrote it; a gradient that does not exist is an error."""
 
 from __future__ import annotations
 
@@ -11,7 +12,7 @@ from torch.utils._python_dispatch import TorchDispatchMode
 
 from dpt_b200._device import StatusWord
 from dpt_b200.geometry import RigidTransform
-from dpt_b200.torch import Projector
+from dpt_b200.torch import Projector, _projection_ops
 from scenes import cone_scene
 
 ANCHORS = [None, RigidTransform(translation_mm=(1.0, -2.0, 3.0))]
@@ -141,3 +142,16 @@ def test_status_word_a_graph_was_given_is_read_at_every_checkpoint(word):
     assert word.pending(side, reset=True) == 8
     word.copies.clear()
     assert word.pending(side) == 0 and word.copies == [2]
+
+
+def test_every_operator_is_compliant_and_refuses_a_second_derivative():
+    for name in ("project", "project_vjp", "project_out", "compose_pose", "compose_pose_vjp"):
+        assert torch.Tag.pt2_compliant_tag in getattr(torch.ops.dpt, name).default.tags
+    grid, geometry, _ = cone_scene(views=2)
+    value = _projection_ops.configuration(grid, geometry, 4, "float32")
+    field = torch.empty(grid.shape, device="meta", requires_grad=True)
+    poses = torch.empty((2, 12), dtype=torch.float64, device="meta")
+    cotangent = torch.empty(geometry.shape, device="meta", requires_grad=True)
+    gradient, _ = torch.ops.dpt.project_vjp(field, poses, cotangent, value, True, False)
+    with pytest.raises(RuntimeError, match="derivative"):
+        gradient.sum().backward()
