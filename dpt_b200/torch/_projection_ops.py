@@ -334,7 +334,9 @@ def _compose_vjp_fake(poses, tangent, cotangent):
 
 
 def _compose_setup(ctx, inputs, output):
-    ctx.save_for_backward(output, inputs[1])
+    # a copy of the tangent: a caller may update its pose in place before the backward, as Torch's
+    # reverse pass of compose_pose, which saves the exponential instead, lets it
+    ctx.save_for_backward(output, inputs[1].clone())
 
 
 def _compose_backward(ctx, cotangent):

@@ -102,3 +102,16 @@ def test_an_error_of_a_replayed_graph_reaches_the_next_operator():
     value.backward()
     assert float(mu.grad.abs().sum()) > 0
     del graph
+
+
+def test_a_pose_updated_in_place_before_the_backward_keeps_its_gradient():
+    grid, geometry, values = cone_scene(views=3)
+    field = torch.tensor(values, dtype=torch.float32, device=DEVICE)
+    projector = Projector(grid=grid, geometry=geometry, samples_per_ray=64)
+    poses = [torch.full((3, 6), 0.01, dtype=torch.float64, device=DEVICE, requires_grad=True) for _ in range(2)]
+    images = [projector(field, pose) for pose in poses]
+    with torch.no_grad():
+        poses[1].add_(0.5)
+    for image in images:
+        image.sum().backward()
+    torch.testing.assert_close(poses[1].grad, poses[0].grad, rtol=1e-12, atol=0)

@@ -155,3 +155,13 @@ def test_every_operator_is_compliant_and_refuses_a_second_derivative():
     gradient, _ = torch.ops.dpt.project_vjp(field, poses, cotangent, value, True, False)
     with pytest.raises(RuntimeError, match="derivative"):
         gradient.sum().backward()
+
+
+def test_a_tangent_updated_in_place_before_the_backward_is_accepted():
+    anchor = torch.tensor(RigidTransform().packed(), dtype=torch.float64)
+    tangent = torch.full((6,), 0.1, dtype=torch.float64, requires_grad=True)
+    poses = _projection_ops.compose_fixed_anchor(anchor, tangent)
+    saved = poses.grad_fn.saved_tensors[1]
+    with torch.no_grad():
+        tangent.add_(1.0)
+    assert poses.grad_fn.saved_tensors[1].tolist() == saved.tolist() == [0.1] * 6
