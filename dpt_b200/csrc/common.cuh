@@ -1327,6 +1327,8 @@ __device__ __forceinline__ void corner_weights2(f32x2 fx, f32x2 fy, f32x2 fz, f3
 // Scatter increments of two samples, ((factor f0) f1) f2 per corner: factor times the corner
 // weights with the factor taken into the x pair (14 products for the 20 of weights then
 // scaling, as many roundings each), the last product flushing results below the normal range.
+// The joint volume + pose pass, which has the weights, forms factor ((f0 f1) f2) as the reference
+// does: an increment of the two passes may differ in its last bit.
 __device__ __forceinline__ void scatter_increments2(f32x2 factor, f32x2 fx, f32x2 fy, f32x2 fz, f32x2* inc)
 {
     const f32x2 one = splat2(1.0f);
@@ -1341,6 +1343,16 @@ __device__ __forceinline__ void scatter_increments2(f32x2 factor, f32x2 fx, f32x
     inc[5] = mul_ftz2(p10, fz);
     inc[6] = mul_ftz2(p01, fz);
     inc[7] = mul_ftz2(p11, fz);
+}
+
+// The same of one sample, rounded alike.
+__device__ __forceinline__ void scatter_increments(float factor, float fx, float fy, float fz, float* inc)
+{
+    const float ay = 1.0f - fy, az = 1.0f - fz;
+    const float px = factor * fx, qx = factor * (1.0f - fx);
+    const float plane[4] = {qx * ay, px * ay, qx * fy, px * fy};
+#pragma unroll
+    for (int c = 0; c < 8; ++c) inc[c] = mul_ftz(plane[c & 3], (c & 4) ? fz : az);
 }
 
 // The twelve corner differences of one cell that its interior slopes combine: along x

@@ -323,18 +323,26 @@ __global__ void __launch_bounds__(kVjpBlock, vjp_min_blocks<kArith, kVol, kPose,
                         if (kVol) {
                             if (in) {
                                 if constexpr (kBounded) {
-                                    // a run's first increments start its sums (0 + x differs
-                                    // from x only for x = -0, and a -0 run sum leaves the
-                                    // +0-initialised accumulator slot exactly as +0 does):
-                                    // 234.8 ms per full-scan volume pass, 235.9 with zeroing
+                                    // the increments of the pairs, so that a ray's sums do not
+                                    // depend on the loops its warp runs; a run's first ones start
+                                    // its sums (0 + x differs from x only for x = -0, and a -0 run
+                                    // sum leaves the +0-initialised accumulator slot exactly as +0
+                                    // does)
+                                    float inc[8];
+                                    if constexpr (kPose) {
+#pragma unroll
+                                        for (int c = 0; c < 8; ++c) inc[c] = mul_ftz(vf, w[c]);
+                                    } else {
+                                        scatter_increments(vf, X.fraction, Y.fraction, Z.fraction, inc);
+                                    }
                                     if (cell != pending) {
                                         if (pending >= 0) flush_run(pending, cs);
                                         pending = cell;
 #pragma unroll
-                                        for (int c = 0; c < 8; ++c) cs[c] = mul_ftz(vf, w[c]);
+                                        for (int c = 0; c < 8; ++c) cs[c] = inc[c];
                                     } else {
 #pragma unroll
-                                        for (int c = 0; c < 8; ++c) cs[c] = cs[c] + mul_ftz(vf, w[c]);
+                                        for (int c = 0; c < 8; ++c) cs[c] = cs[c] + inc[c];
                                     }
                                 } else {
                                     // increments that may be non-finite or large: each one is

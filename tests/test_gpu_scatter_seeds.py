@@ -7,6 +7,8 @@ import numpy as np
 import pytest
 import torch
 
+from dpt_b200.geometry import BatchedGeometry, ParallelGeometry
+from dpt_b200.phantoms import centred_grid
 from dpt_b200.plan import plan_rays
 from dpt_b200.projection import ProjectionSpec, ProjectionWorkspace
 from oracle import oracle as O
@@ -61,3 +63,31 @@ def test_seeds_of_every_size_in_one_warp_match_the_oracle():
         assert own.sum() > 100
         assert np.linalg.norm(actual[own] / part.max() - part[own] / part.max()) <= 2e-6 * np.linalg.norm(part[own] / part.max())
     assert not actual[touched == 0].any()
+
+
+@pytest.mark.parametrize("sampling", ["float32", "float64"])
+def test_a_rays_increments_do_not_depend_on_its_warp(sampling):
+    """A warp with a ray along a face marches every sample in one clamped loop, without one margin
+    samples and interior pairs apart: both form the same sums, bit for bit."""
+    grid = centred_grid((40, 44, 48), (1.0, 1.0, 1.0))
+    # along x; the last column 0.27 beyond the outer voxel centres, inside the half-cell support
+    panel = ParallelGeometry((40.0, 21.77 - 7 * 5.93, -12.31), (1.0, 0.0, 0.0), 80.0, (0.0, 1.0, 0.0), (0.0, 0.0, 1.0),
+                             (5.93, 7.07), (4, 8))
+    precision = "float64" if sampling == "float64" else "float32"
+    ws = ProjectionWorkspace(plan_rays(grid, BatchedGeometry((panel,))),
+                             ProjectionSpec(SAMPLES, precision=precision, sampling_precision=sampling), "cuda:0")
+    dtype = torch.float64 if precision == "float64" else torch.float32
+    field = torch.rand(grid.shape, device="cuda:0")
+    pose = torch.tensor([[1.0, 0, 0, 0, 1, 0, 0, 0, 1, 0, 0, 0]], dtype=torch.float64, device="cuda:0")
+    seeds = torch.linspace(0.3, 1.7, 32, dtype=dtype, device="cuda:0").reshape(ws.plan.image_shape)
+    together, _ = ws.vjp(field, pose, seeds, volume=True, pose=None)
+    apart = torch.zeros_like(together)
+    for ray in range(32):
+        one = torch.zeros_like(seeds)
+        one.view(-1)[ray] = seeds.view(-1)[ray]
+        alone, _ = ws.vjp(field, pose, one, volume=True, pose=None)
+        # 48 voxels along x by two in z and, off the face, two in y, of no other ray
+        assert not bool(((alone != 0) & (apart != 0)).any())
+        assert int((alone != 0).sum()) == (96 if ray % 8 == 7 else 192)
+        apart += alone
+    torch.testing.assert_close(together, apart, rtol=0, atol=0)
