@@ -176,6 +176,12 @@ def _on(device: torch.device):
     return contextlib.nullcontext() if torch.cuda.current_device() == device.index else torch.cuda.device(device)
 
 
+def _free_bytes(device: torch.device) -> int:
+    """Device memory a new tensor can take: free on the device or unused in Torch's pool."""
+    free, _ = torch.cuda.mem_get_info(device)
+    return free + torch.cuda.memory_reserved(device) - torch.cuda.memory_allocated(device)
+
+
 class FieldCopies:
     """Field copies (the replicated or polynomial sampling layout) shared by every workspace
     on one device that samples the same field with the same layout, so that many request
@@ -287,6 +293,7 @@ class ProjectionWorkspace:
         self._partials: torch.Tensor | None = None
         self._moments: torch.Tensor | None = None
         self._moments_for: tuple | None = None
+        self._moments_refused = False
         # Optional instrumentation: a list receiving (name, view_begin, view_count,
         # start_event, end_event) per C-ABI call, and a count of C-ABI calls.
         self.launch_log: list | None = None
@@ -309,6 +316,7 @@ class ProjectionWorkspace:
         self._packed = self._packed_for = None
         self._accumulator = self._total = self._partials = None
         self._moments = self._moments_for = None
+        self._moments_refused = False
 
     def _bytes(self, size: int) -> torch.Tensor:
         # 256-byte aligned storage from the caching allocator
@@ -453,6 +461,8 @@ class ProjectionWorkspace:
     # ------------------------------------------------------------ compute
     # Largest stored pose moments (FP32 words) a workspace keeps between a forward and its VJP.
     MOMENT_BYTES_LIMIT = 16 << 30
+    # The strict FP64 ones leave at least seven eighths of what is free to the caller.
+    MOMENT_FREE_SHARE = 8
 
     def _moment_bytes(self) -> int:
         """Bytes of this workspace's stored pose moments (FP32 words, FP64 for strict FP64)."""
@@ -479,19 +489,27 @@ class ProjectionWorkspace:
         return self.spec.arith in (N.ARITH_F32, N.ARITH_F64) and self.moments_supported()
 
     def _allocate_moments(self) -> bool:
-        """Hold storage for the pose moments; False where they are not supported, or the strict
-        FP64 ones (twice the words of FP32) do not fit the device beside the caller's tensors."""
-        if not self.moments_supported():
+        """Hold storage for the pose moments; False where they are not supported, or for the strict
+        FP64 ones (72 bytes per ray that a step without them does not need) where they would take
+        more than a MOMENT_FREE_SHARE-th of the device's free memory.  A refusal stays until
+        ``release_scratch``: each failing allocation would empty Torch's pool."""
+        if not self.moments_supported() or self._moments_refused:
             return False
         size = self._moment_bytes()
         wide = self.spec.arith == N.ARITH_F64
         if self._moments is None or self._moments.numel() * self._moments.element_size() < size:
+            if wide and torch.cuda.is_current_stream_capturing():
+                return False  # decided outside captures
             try:
+                if wide and size * self.MOMENT_FREE_SHARE > _free_bytes(self.device):
+                    self._moments_refused = True
+                    return False
                 self._moments = torch.empty(size // (8 if wide else 4), device=self.device,
                                             dtype=torch.float64 if wide else torch.float32)
             except torch.OutOfMemoryError:
                 if not wide:
                     raise
+                self._moments_refused = True
                 return False
         return True
 

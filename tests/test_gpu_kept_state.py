@@ -8,7 +8,7 @@ import torch
 
 from dpt_b200.contracts import NumericalError, TrialDomainError
 from dpt_b200.objectives import ObjectiveSpec, evaluate_objective, prepare_objective
-from dpt_b200.torch import Projector
+from dpt_b200.torch import Projector, _projection_ops
 from dpt_b200.torch.operators import objective
 from dpt_b200.transmission import TransmissionSpec, prepare_transmission, transmission_vjp, transmit
 from scenes import cone_scene
@@ -115,3 +115,27 @@ def test_a_pose_updated_in_place_before_the_backward_keeps_its_gradient():
     for image in images:
         image.sum().backward()
     torch.testing.assert_close(poses[1].grad, poses[0].grad, rtol=1e-12, atol=0)
+
+
+def test_strict_fp64_step_without_room_for_its_moments(monkeypatch):
+    """Beside little free memory the step samples twice: no kept moments, the same image and pose
+    gradient, and a volume gradient to FP32 summation order."""
+    grid, geometry, values = cone_scene(views=3)
+    results, held = [], []
+    for free in (None, 1 << 10):
+        _projection_ops.clear_cache()
+        if free is not None:
+            monkeypatch.setattr(torch.cuda, "mem_get_info", lambda device: (free, 1 << 40))
+            monkeypatch.setattr(torch.cuda, "memory_reserved", lambda device: 0)
+            monkeypatch.setattr(torch.cuda, "memory_allocated", lambda device: 0)
+        field = torch.tensor(values, dtype=torch.float32, device=DEVICE, requires_grad=True)
+        pose = torch.full((3, 6), 0.01, dtype=torch.float64, device=DEVICE, requires_grad=True)
+        image = Projector(grid=grid, geometry=geometry, samples_per_ray=64, precision="fp64")(field, pose)
+        image.sum().backward()
+        results.append((image.detach(), pose.grad, field.grad))
+        held.append([ws._moments is not None for ws in _projection_ops._CACHE.values()])
+    assert held == [[True], [False]]
+    torch.testing.assert_close(results[1][0], results[0][0], rtol=0, atol=0)
+    torch.testing.assert_close(results[1][1], results[0][1], rtol=1e-9, atol=1e-12)
+    assert float((results[1][2] - results[0][2]).norm()) <= 2e-6 * float(results[0][2].norm())
+    _projection_ops.clear_cache()

@@ -12,6 +12,7 @@ from torch.utils._python_dispatch import TorchDispatchMode
 
 from dpt_b200._device import StatusWord
 from dpt_b200.geometry import RigidTransform
+from dpt_b200.projection import ProjectionSpec, ProjectionWorkspace
 from dpt_b200.torch import Projector, _projection_ops
 from scenes import cone_scene
 
@@ -165,3 +166,26 @@ def test_a_tangent_updated_in_place_before_the_backward_is_accepted():
     with torch.no_grad():
         tangent.add_(1.0)
     assert poses.grad_fn.saved_tensors[1].tolist() == saved.tolist() == [0.1] * 6
+
+
+@pytest.mark.parametrize("free,allocations", [(1000, 0), (10000, 1)])
+def test_moments_that_do_not_fit_are_refused_once(monkeypatch, free, allocations):
+    """Strict FP64 moments of 800 bytes: beside 1000 free bytes none is tried, and one allocation
+    that fails all the same is not repeated at every step."""
+    workspace = ProjectionWorkspace.__new__(ProjectionWorkspace)
+    workspace.spec = ProjectionSpec(4, precision="float64", sampling_precision="float64")
+    workspace.device, workspace._moments, workspace._moments_refused = torch.device("cuda:0"), None, False
+    monkeypatch.setattr(ProjectionWorkspace, "_moment_bytes", lambda self: 800)
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    monkeypatch.setattr(torch.cuda, "mem_get_info", lambda device: (free, 1 << 40))
+    monkeypatch.setattr(torch.cuda, "memory_reserved", lambda device: 0)
+    monkeypatch.setattr(torch.cuda, "memory_allocated", lambda device: 0)
+    tried = []
+
+    def empty(*args, **kwargs):
+        tried.append(args)
+        raise torch.OutOfMemoryError
+
+    monkeypatch.setattr(torch, "empty", empty)
+    assert [workspace._allocate_moments() for _ in range(3)] == [False] * 3
+    assert len(tried) == allocations
