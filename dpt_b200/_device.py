@@ -59,21 +59,21 @@ class StatusWord:
         with current(stream, self.device):
             return torch.cuda.is_current_stream_capturing()
 
-    def _count(self, stream: torch.cuda.Stream) -> None:
+    def _count(self, handle: int) -> None:
         with self._lock:
-            self._unread[stream.cuda_stream] = self._unread.get(stream.cuda_stream, 0) + 1
+            self._unread[handle] = self._unread.get(handle, 0) + 1
 
-    @contextlib.contextmanager
-    def launch(self, stream: torch.cuda.Stream):
-        """The word's address for one call that queues its work on `stream` in this block.  Under
-        capture every replay of the graph may report, unseen from here."""
+    def launch(self, stream: torch.cuda.Stream, what: str, function, *arguments) -> None:
+        """Queue the C-ABI call ``function(*arguments, word, stream)``.  Under capture every replay of
+        the graph may report, unseen from here."""
         if self._capturing(stream):
             self._untracked = True
-        self._count(stream)
+        handle = stream.cuda_stream
+        self._count(handle)
         try:
-            yield self.word.data_ptr()
+            call(function(*arguments, self.word.data_ptr(), handle), what)
         finally:
-            self._count(stream)
+            self._count(handle)
 
     def pending(self, stream: torch.cuda.Stream, *, reset: bool = False) -> int:
         """``read`` where a launch may have reported since the last clean read, else 0 without

@@ -122,10 +122,10 @@ class ObjectiveWorkspace:
         self._raise(self.status.pending(stream))
         if size:
             dtype = N.F64 if prediction is not None and prediction.dtype == torch.float64 else N.F32
-            with self.status.launch(stream) as status:
-                D.call(N.library().dpt_b200_objective_check(
-                    D.ptr(prediction), dtype, observation.data_ptr(), D.ptr(weights), D.ptr(valid), size,
-                    self.spec.code, int(self.spec.integer_counts), status, stream.cuda_stream), "objective check")
+            self.status.launch(
+                stream, "objective check", N.library().dpt_b200_objective_check, D.ptr(prediction), dtype,
+                observation.data_ptr(), D.ptr(weights), D.ptr(valid), size, self.spec.code,
+                int(self.spec.integer_counts))
         self._raise(self.status.read(stream))
 
     def validate_observation(self, observation: torch.Tensor, *, weights: torch.Tensor | None = None,
@@ -154,11 +154,10 @@ def _run(workspace: ObjectiveWorkspace, stream, prediction, observation, weights
          wide: bool, seed_scale: float, seed, loss) -> None:
     normalisation = 1.0 / size if workspace.spec.reduction == "mean" and size else 1.0
     dtype = N.F64 if prediction.dtype == torch.float64 else N.F32
-    with workspace.status.launch(stream) as status:
-        D.call(N.library().dpt_b200_objective(
-            prediction.data_ptr(), dtype, int(wide), observation.data_ptr(), D.ptr(weights), D.ptr(valid), size,
-            workspace.spec.code, normalisation, seed_scale, D.ptr(seed), workspace._scratch.data_ptr(), D.ptr(loss),
-            status, stream.cuda_stream), "objective")
+    workspace.status.launch(
+        stream, "objective", N.library().dpt_b200_objective, prediction.data_ptr(), dtype, int(wide),
+        observation.data_ptr(), D.ptr(weights), D.ptr(valid), size, workspace.spec.code, normalisation, seed_scale,
+        D.ptr(seed), workspace._scratch.data_ptr(), D.ptr(loss))
 
 
 def evaluate_objective(prediction: torch.Tensor, observation: torch.Tensor, *, out_loss: torch.Tensor,
@@ -229,9 +228,7 @@ def reduce_objective_components(components: torch.Tensor, *, out_loss: torch.Ten
     D.disjoint([("components", components)], [("out_loss", out_loss)], ContractError)
     if validate:
         workspace.check_status()
-    with workspace.status.launch(launch) as status:
-        D.call(N.library().dpt_b200_reduce_sum(components.data_ptr(), size, workspace._scratch.data_ptr(),
-                                               out_loss.data_ptr(), status, launch.cuda_stream),
-               "reduce_objective_components")
+    workspace.status.launch(launch, "reduce_objective_components", N.library().dpt_b200_reduce_sum,
+                            components.data_ptr(), size, workspace._scratch.data_ptr(), out_loss.data_ptr())
     if validate:
         workspace.check_status()

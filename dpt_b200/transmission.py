@@ -164,9 +164,8 @@ def _check_values(workspace: TransmissionWorkspace, stream: torch.cuda.Stream,
     lib = N.library()
     for name, array, rule in arrays:
         if array is not None and array.numel():
-            with workspace.status.launch(stream) as status:
-                D.call(lib.dpt_b200_check_values(array.data_ptr(), array.numel(), _RULES[rule], status,
-                                                 stream.cuda_stream), f"check {name}")
+            workspace.status.launch(stream, f"check {name}", lib.dpt_b200_check_values, array.data_ptr(),
+                                    array.numel(), _RULES[rule])
     code = workspace.status.read(stream)
     if not code:
         return
@@ -264,11 +263,10 @@ def transmission_vjp(L: torch.Tensor, n0: float | torch.Tensor | None = None, *,
     D.disjoint(reads, writes, TransmissionError)
     if validate:
         _check_values(workspace, launch, rules)
-    with workspace.status.launch(launch) as status:
-        D.call(N.library().dpt_b200_transmit_vjp(
-            L.data_ptr(), count, _BEAM_MODES[workspace.spec.beam], D.ptr(beam), scalar, *(D.ptr(s) for s in seeds),
-            D.ptr(out_grad_L), D.ptr(out_grad_n0), D.ptr(workspace._scratch), int(_accumulate), status,
-            launch.cuda_stream), "transmission_vjp")
+    workspace.status.launch(
+        launch, "transmission_vjp", N.library().dpt_b200_transmit_vjp, L.data_ptr(), count,
+        _BEAM_MODES[workspace.spec.beam], D.ptr(beam), scalar, *(D.ptr(s) for s in seeds), D.ptr(out_grad_L),
+        D.ptr(out_grad_n0), D.ptr(workspace._scratch), int(_accumulate))
     if validate:
         workspace.check_status()
 
@@ -301,9 +299,7 @@ def optical_depth_from_removed_vjp(delta: torch.Tensor, cotangent: torch.Tensor,
     if validate:
         _check_values(workspace, launch, [("delta", delta, "decrement_domain"),
                                           ("cotangent", cotangent, "finite_seed")])
-    with workspace.status.launch(launch) as status:
-        D.call(N.library().dpt_b200_depth_from_removed_vjp(delta.data_ptr(), cotangent.data_ptr(), count,
-                                                           out_grad_delta.data_ptr(), int(_accumulate), status,
-                                                           launch.cuda_stream), "optical_depth_from_removed_vjp")
+    workspace.status.launch(launch, "optical_depth_from_removed_vjp", N.library().dpt_b200_depth_from_removed_vjp,
+                            delta.data_ptr(), cotangent.data_ptr(), count, out_grad_delta.data_ptr(), int(_accumulate))
     if validate:
         workspace.check_status()

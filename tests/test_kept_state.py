@@ -104,11 +104,16 @@ def word(monkeypatch):
     return status
 
 
+def report(word, stream, address, handle) -> int:
+    """A C-ABI call that reports 8."""
+    assert (address, handle) == (word.word.data_ptr(), stream.cuda_stream)
+    word.word.fill_(8)
+    return 0
+
+
 def test_status_word_is_read_on_the_stream_that_writes_it(word):
     side = FakeStream(2)
-    with word.launch(side) as address:
-        assert address == word.word.data_ptr()
-    word.word.fill_(8)
+    word.launch(side, "report", lambda address, stream: report(word, side, address, stream))
     assert word.read(side) == 8 and word.pending(side) == 8  # sticky until reset
     assert word.pending(side, reset=True) == 8 and word.pending(side) == 0
     assert int(word.word) == 0 and word.copies == [2, 2, 2]
@@ -117,11 +122,10 @@ def test_status_word_is_read_on_the_stream_that_writes_it(word):
 def test_status_word_stays_pending_until_its_own_stream_was_read_clean(word):
     side, other = FakeStream(2), FakeStream(3)
     assert word.pending(side) == 0 and word.copies == []  # no launch: no wait
-    with word.launch(side):
-        word.read(side)  # another thread's read before the launch is queued
+    # another thread's read before the launch is queued
+    word.launch(side, "nothing", lambda address, stream: word.read(side) and 1)
     assert word.pending(side) == 0 and word.copies == [2, 2]
-    with word.launch(side):
-        pass
+    word.launch(side, "nothing", lambda address, stream: 0)
     word.read(other)  # ordered after another stream only
     word.clear(other)
     word.word.fill_(2)  # the launch reports now
@@ -136,8 +140,7 @@ def test_status_word_stays_pending_until_its_own_stream_was_read_clean(word):
 def test_status_word_a_graph_was_given_is_read_at_every_checkpoint(word):
     side, capturing = FakeStream(2), FakeStream(CAPTURING)
     assert word.pending(capturing) == 0 and word.copies == [CAPTURING]  # where a real one refuses
-    with word.launch(capturing):
-        pass
+    word.launch(capturing, "nothing", lambda address, stream: 0)
     assert word.read(capturing) == 0 and word.read(side) == 0
     word.word.fill_(8)  # a replay reports
     assert word.pending(side, reset=True) == 8
