@@ -38,3 +38,9 @@ def test_tangent_gradient_equals_the_reverse_pass_of_the_chart(anchors, tangents
     got, = torch.autograd.grad(actual, actual_in, cotangent)
     assert got.shape == want.shape
     assert float((got - want).norm()) <= 1e-12 * float(want.norm())
+
+
+@pytest.mark.parametrize("angle", [3.2, 6.283184307, 6.283185307179586, 7.0, 20.0])
+def test_tangent_gradient_beyond_a_half_turn(angle):
+    """The closed form up to three turns, at the same bar: its cancellation only shrinks with theta."""
+    test_tangent_gradient_equals_the_reverse_pass_of_the_chart((300, 12), (300, 6), angle)
