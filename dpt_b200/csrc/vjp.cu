@@ -248,8 +248,8 @@ __global__ void __launch_bounds__(kVjpBlock, vjp_min_blocks<kArith, kVol, kPose,
                     // Every increment is at most |vf| in magnitude, and rounding at most doubles
                     // what one adds to a sum: a run of up to 2^31 of them stays below 4.3e37.
                     // Residuals in counts are in here too: at seeds of 100, 32 views of the 256^3 /
-                    // 512^2 / S = 1024 scan take 16.2 ms for the volume gradient and 33.7 with the pose's, where
-                    // the loop that tests each increment took 48.1 and 102.9.
+                    // 512^2 / S = 1024 scan take 16.1 ms for the volume gradient and 33.6 with the
+                    // pose's, where the loop that tests each increment took 48.1 and 102.9.
                     const bool bounded = fabsf(vf) <= 1e28f;
                     float mean = 0.0f, dO[3] = {0.0f, 0.0f, 0.0f}, dD[3] = {0.0f, 0.0f, 0.0f};
                     float sl = 0.0f, su = 0.0f;
@@ -383,12 +383,14 @@ __global__ void __launch_bounds__(kVjpBlock, vjp_min_blocks<kArith, kVol, kPose,
                     // whose clamps and slope masks then apply), lane-wise where the arithmetic is
                     // (see "packed FP32 pairs" in common.cuh); the serial sums take sample i,
                     // then sample i + 1, so every moment, increment and run sum is the value
-                    // the two visits form.  `ip` holds (i + 0.5, i + 1.5).  Positions and
+                    // the two visits form (increments of the volume-only scatter round as
+                    // scatter_increments does).  `ip` holds (i + 0.5, i + 1.5).  Positions and
                     // coordinates stay scalar (a packed operand of a per-ray value takes two
                     // registers).  The corners reload, and a finished run flushes, under a
                     // predicate instead of a branch: 32 views of the 256^3 / 512^2 / S = 1024
-                    // scan take 32.8 ms jointly (51.2 before), 23.6 storing the moments (25.2),
-                    // 15.5 scattering (16.3); 512^3 at 0.5 mm, 16 views: 14.4 (15.6) and 29.0 (31.3).
+                    // scan take 32.6 ms jointly (51.5 before), 23.5 storing the moments (25.3),
+                    // 15.1 scattering (16.2); 16 views of a 512^3 volume at 0.5 mm 38.6 (45.7),
+                    // 17.1 (18.2) and 34.9 (37.7).
                     auto visit_pair = [&](int i, f32x2 ip, auto pow2_tag, auto clamped_tag) {
                         constexpr bool kClamped = decltype(clamped_tag)::value;
                         const float q0 = fmaf(lo2(ip), step, iv.lower), q1 = fmaf(hi2(ip), step, iv.lower);

@@ -459,7 +459,7 @@ class ProjectionWorkspace:
             raise first
 
     # ------------------------------------------------------------ compute
-    # Largest stored pose moments (FP32 words) a workspace keeps between a forward and its VJP.
+    # Largest stored pose moments a workspace keeps between a forward and its VJP.
     MOMENT_BYTES_LIMIT = 16 << 30
     # The strict FP64 ones leave at least seven eighths of what is free to the caller.
     MOMENT_FREE_SHARE = 8
@@ -481,11 +481,12 @@ class ProjectionWorkspace:
     def moments_preferred(self) -> bool:
         """Whether a training step should store the pose moments in its forward (and run the
         volume-only scatter in its VJP) rather than run a plain forward and a joint volume +
-        pose VJP.  Measured on 64 views of the 256^3 / 512^2 / S = 1024 full scan: FP32
-        arithmetic 101.1 ms split against 114.5 ms joint; the compensated form 65.4 ms split
-        against 64.2 ms joint (its moment-storing forward costs more than the pose terms add
-        to a pass bound by its scatter).  Strict FP64, 16 views:
-        forward and VJP 31 ms split, 47 ms joint."""
+        pose VJP.  Forward and VJP of 16, 64 and 360 views of the 256^3 / 512^2 / S = 1024 scan,
+        split against joint: FP32 arithmetic 20.0 / 23.0, 80.4 / 91.7 and 455.7 / 515.4 ms; strict
+        FP64 32.8 / 44.9 and 130.2 / 179.2 ms; the compensated form 12.7 / 13.0, 51.3 / 51.2 and
+        305.5 / 297.6 ms, so it stays joint for the large scans (and holds no moments).  Under two
+        samples per cell the order turns: 16 views of 512^3 at 0.5 mm take 55.4 / 52.9 ms in FP32
+        and 53.8 / 60.5 compensated."""
         return self.spec.arith in (N.ARITH_F32, N.ARITH_F64) and self.moments_supported()
 
     def _allocate_moments(self) -> bool:
