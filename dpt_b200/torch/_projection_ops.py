@@ -44,7 +44,12 @@ from .geometry import compose_pose
 _CACHE_LIMIT = 8
 _CACHE: OrderedDict[tuple, ProjectionWorkspace] = OrderedDict()
 _CACHE_LOCK = RLock()
-_TAGS = (torch.Tag.cudagraph_unsafe,)  # custom_op adds pt2_compliant_tag
+_TAGS = (torch.Tag.cudagraph_unsafe,)
+# CUDA kernels of the operators below without the wrapper custom_op puts around a body: it costs 20 us
+# a call, a fifth of a small forward (8 views of 64^2).  (None first: on a reload the kernels of the
+# module before go with their library.)
+_CUDA = None
+_CUDA = torch.library.Library("dpt", "IMPL")
 _KINDS = {DetectorGeometry: "cone", ParallelGeometry: "parallel", CurvedDetectorGeometry: "curved"}
 _CONSTRUCTORS = {"cone": DetectorGeometry, "parallel": ParallelGeometry, "curved": CurvedDetectorGeometry}
 _FIELD_DTYPES = (torch.float32, torch.float16, torch.bfloat16)
@@ -183,20 +188,17 @@ def _forward(field, poses, value, active_volume, active_pose, out=None):
                              moments=active_pose and out is None and entry.moments_preferred())
 
 
-def _functional(name: str, schema: str, body) -> torch._ops.OpOverload:
-    """The operator ``dpt::name`` of a body that returns new tensors.  Defined through the library
-    directly: the wrapper ``custom_op`` puts around a body costs 20 us a call, a fifth of a small
-    forward (8 views of 64^2)."""
-    torch.library.define(f"dpt::{name}", schema, tags=(torch.Tag.pt2_compliant_tag, *_TAGS))
-    torch.library.impl(f"dpt::{name}", "default", body)
-    return getattr(torch.ops.dpt, name).default
+@torch.library.custom_op("dpt::project", mutates_args=(), tags=_TAGS)
+def project(
+    field: torch.Tensor, poses: torch.Tensor, value: str, active_volume: bool, active_pose: bool
+) -> torch.Tensor:
+    return _forward(field, poses, value, active_volume, active_pose)
 
 
-project = _functional(
-    "project", "(Tensor field, Tensor poses, str value, bool active_volume, bool active_pose) -> Tensor", _forward)
+_CUDA.impl("project", _forward, "CUDA")
 
 
-@torch.library.register_fake("dpt::project")
+@project.register_fake
 def _project_fake(field, poses, value, active_volume, active_pose):
     shape, dtype = metadata(field, poses, value)
     return torch.empty(shape, dtype=dtype, device=field.device)
@@ -231,13 +233,22 @@ def _project_vjp(
     return gradient, pose_gradient
 
 
-project_vjp = _functional(
-    "project_vjp",
-    "(Tensor field, Tensor poses, Tensor cotangent, str value, bool active_volume, bool active_pose)"
-    " -> (Tensor, Tensor)", _project_vjp)
+@torch.library.custom_op("dpt::project_vjp", mutates_args=(), tags=_TAGS)
+def project_vjp(
+    field: torch.Tensor,
+    poses: torch.Tensor,
+    cotangent: torch.Tensor,
+    value: str,
+    active_volume: bool,
+    active_pose: bool,
+) -> tuple[torch.Tensor, torch.Tensor]:
+    return _project_vjp(field, poses, cotangent, value, active_volume, active_pose)
 
 
-@torch.library.register_fake("dpt::project_vjp")
+_CUDA.impl("project_vjp", _project_vjp, "CUDA")
+
+
+@project_vjp.register_fake
 def _vjp_fake(field, poses, cotangent, value, active_volume, active_pose):
     shape, dtype = metadata(field, poses, value)
     if tuple(cotangent.shape) != shape or cotangent.dtype != dtype or cotangent.device != field.device:
@@ -246,14 +257,6 @@ def _vjp_fake(field, poses, cotangent, value, active_volume, active_pose):
         field.new_empty(field.shape if active_volume else (0,)),
         poses.new_empty(poses.shape if active_pose else (0,)),
     )
-
-
-def _vjp_backward(ctx, *cotangents):
-    raise RuntimeError("dpt::project_vjp has no derivative formula: projection gradients are first order")
-
-
-# without a formula of its own the operator would only warn and leave its inputs without a gradient
-torch.library.register_autograd("dpt::project_vjp", _vjp_backward)
 
 
 def _setup_context(ctx, inputs, output):
@@ -279,7 +282,7 @@ def _backward(ctx, cotangent):
     )
 
 
-torch.library.register_autograd("dpt::project", _backward, setup_context=_setup_context)
+project.register_autograd(_backward, setup_context=_setup_context)
 
 
 @torch.library.custom_op("dpt::project_out", mutates_args={"out"}, tags=_TAGS)
