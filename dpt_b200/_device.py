@@ -36,8 +36,8 @@ class StatusWord:
     The word remembers on which streams launches may have reported since that stream's last clean
     read, so that a checkpoint with nothing to read needs no wait (``pending``; a checked likelihood
     step of 23.6 M pixels has 15 checkpoints, 8 of them with nothing to read).  Several threads may
-    share it: a launch counts when it begins and again when it is queued, and a read clears only
-    what was counted before its copy was queued and has not moved since."""
+    share it: a launch leaves a mark once it is queued, and a read clears only the mark it found
+    before its copy was queued."""
 
     def __init__(self, device: torch.device) -> None:
         self.device = device
@@ -45,7 +45,7 @@ class StatusWord:
         self.word = torch.tensor([0], dtype=torch.int32, device=device)
         self.host = torch.zeros(1, dtype=torch.int32, pin_memory=True)
         self._lock = threading.Lock()
-        self._unread: dict[int, int] = {}  # stream handle -> count of launches since a clean read
+        self._unread: dict[int, object] = {}  # stream handle -> mark of its last launch, until read clean
         self._untracked = False  # whether the word's address was given away, or captured
 
     @property
@@ -55,13 +55,14 @@ class StatusWord:
         self._untracked = True
         return self.word.data_ptr()
 
-    def _capturing(self, stream: torch.cuda.Stream) -> bool:
-        with current(stream, self.device):
-            return torch.cuda.is_current_stream_capturing()
+    def _on(self, stream: torch.cuda.Stream):
+        """``torch.cuda.stream(stream)``, or nothing where it is the current stream already."""
+        same = torch._C._cuda_getCurrentRawStream(self.device.index) == stream.cuda_stream
+        return _HERE if same else torch.cuda.stream(stream)
 
-    def _count(self, handle: int) -> None:
-        with self._lock:
-            self._unread[handle] = self._unread.get(handle, 0) + 1
+    def _capturing(self, stream: torch.cuda.Stream) -> bool:
+        with self._on(stream):
+            return torch.cuda.is_current_stream_capturing()
 
     def launch(self, stream: torch.cuda.Stream, what: str, function, *arguments) -> None:
         """Queue the C-ABI call ``function(*arguments, word, stream)``.  Under capture every replay of
@@ -69,11 +70,11 @@ class StatusWord:
         if self._capturing(stream):
             self._untracked = True
         handle = stream.cuda_stream
-        self._count(handle)
         try:
             call(function(*arguments, self.word.data_ptr(), handle), what)
         finally:
-            self._count(handle)
+            with self._lock:
+                self._unread[handle] = object()
 
     def pending(self, stream: torch.cuda.Stream, *, reset: bool = False) -> int:
         """``read`` where a launch may have reported since the last clean read, else 0 without
@@ -85,29 +86,25 @@ class StatusWord:
     def read(self, stream: torch.cuda.Stream, *, reset: bool = False) -> int:
         """Synchronise `stream` and return the word; with `reset`, clear it afterwards."""
         handle = stream.cuda_stream
-        with self._lock:
-            seen = self._unread.get(handle)
-        with current(stream, self.device):
+        seen = self._unread.get(handle)
+        with self._on(stream):
             self.host.copy_(self.word, non_blocking=True)
             stream.synchronize()
             code = int(self.host[0])
             if reset and code:
                 self.word.zero_()
-        if not code or reset:
+        if seen is not None and (not code or reset):
             with self._lock:
-                if self._unread.get(handle) == seen:
-                    self._unread.pop(handle, None)
+                if self._unread.get(handle) is seen:
+                    del self._unread[handle]
         return code
 
     def clear(self, stream: torch.cuda.Stream) -> None:
-        with current(stream, self.device):
+        with self._on(stream):
             self.word.zero_()
 
 
-def current(stream: torch.cuda.Stream, device: torch.device):
-    """``torch.cuda.stream(stream)``, or nothing where it is the device's current stream already."""
-    same = torch._C._cuda_getCurrentRawStream(device.index) == stream.cuda_stream
-    return contextlib.nullcontext() if same else torch.cuda.stream(stream)
+_HERE = contextlib.nullcontext()
 
 
 def resolve_stream(owned: torch.cuda.Stream | None, requested: torch.cuda.Stream | None,
