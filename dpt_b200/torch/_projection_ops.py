@@ -270,9 +270,11 @@ def _backward(ctx, cotangent):
         raise ContractError("the Torch projection adapter supports first-order derivatives only")
     field, poses = ctx.saved_tensors
     active_volume, active_pose = ctx.needs_input_grad[:2]
-    gradient, pose_gradient = project_vjp(
-        field, poses, cotangent.contiguous(), ctx.configuration, active_volume, active_pose
-    )
+    # grad mode is off: there is nothing for the operator's own autograd kernel to record
+    with torch._C._AutoDispatchBelowAutograd():
+        gradient, pose_gradient = project_vjp(
+            field, poses, cotangent.contiguous(), ctx.configuration, active_volume, active_pose
+        )
     return (
         gradient if active_volume else None,
         pose_gradient if active_pose else None,
