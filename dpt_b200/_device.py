@@ -44,6 +44,7 @@ class StatusWord:
         # zeroed by an upload that has ended when it returns: the first reader may use any stream
         self.word = torch.tensor([0], dtype=torch.int32, device=device)
         self.host = torch.zeros(1, dtype=torch.int32, pin_memory=True)
+        self._address = self.word.data_ptr()
         self._lock = threading.Lock()
         self._unread: dict[int, object] = {}  # stream handle -> mark of its last launch, until read clean
         self._untracked = False  # whether the word's address was given away, or captured
@@ -53,15 +54,17 @@ class StatusWord:
         """The word's address for launches this object does not follow: from here on every
         checkpoint reads."""
         self._untracked = True
-        return self.word.data_ptr()
+        return self._address
 
     def _on(self, stream: torch.cuda.Stream):
         """``torch.cuda.stream(stream)``, or nothing where it is the current stream already."""
         same = torch._C._cuda_getCurrentRawStream(self.device.index) == stream.cuda_stream
-        return _HERE if same else torch.cuda.stream(stream)
+        return contextlib.nullcontext() if same else torch.cuda.stream(stream)
 
     def _capturing(self, stream: torch.cuda.Stream) -> bool:
-        with self._on(stream):
+        if torch._C._cuda_getCurrentRawStream(self.device.index) == stream.cuda_stream:
+            return torch.cuda.is_current_stream_capturing()
+        with torch.cuda.stream(stream):
             return torch.cuda.is_current_stream_capturing()
 
     def launch(self, stream: torch.cuda.Stream, what: str, function, *arguments) -> None:
@@ -71,7 +74,7 @@ class StatusWord:
             self._untracked = True
         handle = stream.cuda_stream
         try:
-            call(function(*arguments, self.word.data_ptr(), handle), what)
+            N.check(function(*arguments, self._address, handle), what)
         finally:
             with self._lock:
                 self._unread[handle] = object()
@@ -102,9 +105,6 @@ class StatusWord:
     def clear(self, stream: torch.cuda.Stream) -> None:
         with self._on(stream):
             self.word.zero_()
-
-
-_HERE = contextlib.nullcontext()
 
 
 def resolve_stream(owned: torch.cuda.Stream | None, requested: torch.cuda.Stream | None,

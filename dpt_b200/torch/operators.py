@@ -93,6 +93,7 @@ class _OnWorkspaceStream:
     def __enter__(self) -> _OnWorkspaceStream:
         self.caller = torch.cuda.current_stream(self.device)
         self.separate = self.stream is not None and self.stream.cuda_stream != self.caller.cuda_stream
+        self.launch = self.caller if self.stream is None else self.stream
         if self.separate:
             self.stream.wait_stream(self.caller)
         self.keep(*self.tensors)
@@ -147,8 +148,8 @@ class _TransmissionCall:
             result = torch.empty_like(depth)
             scope.keep(result)
             _transmit(_vector(depth), self.native_beam(beam), **{_KEYWORDS[self.output][0]: _vector(result)},
-                      workspace=self.workspace, stream=self.workspace.stream, validate=self.validate)
-            self.workspace.settle()
+                      workspace=self.workspace, stream=scope.launch, validate=self.validate)
+            self.workspace.settle(scope.launch)
         return result
 
     def backward(self, depth: torch.Tensor, beam, seed: torch.Tensor, wants: tuple[bool, bool]):
@@ -160,8 +161,8 @@ class _TransmissionCall:
             scope.keep(*(g for g in (grad_depth, grad_beam) if g is not None))
             transmission_vjp(_vector(depth), self.native_beam(beam), **{_KEYWORDS[self.output][1]: _vector(seed)},
                              out_grad_L=_vector(grad_depth), out_grad_n0=_vector(grad_beam),
-                             workspace=self.workspace, stream=self.workspace.stream, validate=self.validate)
-            self.workspace.settle()
+                             workspace=self.workspace, stream=scope.launch, validate=self.validate)
+            self.workspace.settle(scope.launch)
         return grad_depth, grad_beam
 
 
@@ -214,13 +215,13 @@ class _ObjectiveCall:
             scope.keep(result)
             evaluate_objective(_vector(prediction), _vector(observation), out_loss=result.reshape(1),
                                weights=_vector(weights), valid=_vector(valid), workspace=self.workspace,
-                               stream=self.workspace.stream, validate=self.validate)
-            self.workspace.settle()
+                               stream=scope.launch, validate=self.validate)
+            self.workspace.settle(scope.launch)
         return result
 
     def gradient(self, prediction, observation, weights, valid, seed: torch.Tensor) -> torch.Tensor:
         with _OnWorkspaceStream(self.workspace, (prediction, observation, weights, valid, seed)) as scope:
-            self.workspace._raise(self.workspace.status.pending(self.workspace._stream()))
+            self.workspace._raise(self.workspace.status.pending(scope.launch))
             scale = float(seed.item())
             if scale - scale != 0.0:  # NaN or infinite
                 raise ContractError("objective cotangent must be finite")
@@ -232,9 +233,9 @@ class _ObjectiveCall:
             scope.keep(gradient)
             objective_seed(_vector(prediction), _vector(observation), scale=scale, out_cotangent=_vector(gradient),
                            weights=_vector(weights), valid=_vector(valid), workspace=self.workspace,
-                           stream=self.workspace.stream, validate=self.validate)
+                           stream=scope.launch, validate=self.validate)
             try:
-                self.workspace.settle()
+                self.workspace.settle(scope.launch)
             except NumericalError as error:
                 # a plain range failure means the FP64 seed overflowed the prediction's dtype;
                 # typed subclasses (an input outside its domain) pass through

@@ -109,9 +109,9 @@ class TransmissionWorkspace:
         """Deliver and reset one completed checkpoint, including reported errors."""
         self._raise(self.status.read(self._stream(), reset=True))
 
-    def settle(self) -> None:
+    def settle(self, stream: torch.cuda.Stream | None = None) -> None:
         """``consume_status`` where a launch may have reported since the last clean checkpoint."""
-        self._raise(self.status.pending(self._stream(), reset=True))
+        self._raise(self.status.pending(self._stream(stream), reset=True))
 
     def warm(self, **_ignored) -> tuple[str, ...]:
         """Kernels are compiled ahead of time: nothing to prepare."""
